@@ -22,7 +22,8 @@ def reference_root() -> str | None:
     root = os.environ.get("ALLEN_REFERENCE_ROOT")
     if root is None:
         root = os.path.join(os.path.dirname(REPO), "reference")
-    return root if os.path.isdir(root) else None
+    # an empty directory of that name holds no sources
+    return root if os.path.isdir(os.path.join(root, "device", "velo")) else None
 
 
 def build_oracle(ref_root: str | None = None, with_reference: bool = True) -> None:
