@@ -54,17 +54,17 @@ namespace velo {
     unsigned designated_stride;           // events e with e % stride == 0 set the bank index
     unsigned* status;
     unsigned smem_blob_bytes;
-    // sorted bank copies for this kernel's neighbour search and the clustering kernel's (null:
-    // full scans): each event takes total_sp words of sp_scratch from the counter sp_alloc
-    // (zeroed before the launch) and records where in sp_base[e] (no_sorted_copy: no room)
-    uint32_t* sp_scratch;
-    unsigned sp_capacity;
-    unsigned* sp_alloc;
-    unsigned* sp_base;
+    // the candidates this kernel finds, for the clustering kernel (null: none are handed over):
+    // each event takes total_sp words of list_scratch from the counter list_alloc (zeroed before
+    // the launch) and records where in list_base[e] (no_candidate_list: no room, or too many)
+    uint32_t* list_scratch;
+    unsigned list_capacity;
+    unsigned* list_alloc;
+    unsigned* list_base;
     WorkQueue queue;
   };
 
-  constexpr unsigned no_sorted_copy = 0xFFFFFFFFu;
+  constexpr unsigned no_candidate_list = 0xFFFFFFFFu;
 
   // ---- masked clustering + phi + sort by phi, one event per CTA ----
   struct ClusterSortParams {
@@ -78,12 +78,9 @@ namespace velo {
     unsigned* module_cluster_num;               // [26 N]     dev_module_cluster_num
     char* sorted_container;                     // [18 T]     dev_sorted_velo_cluster_container
     char* staging;                              // [24 T]     fallback staging for large events
-    const unsigned* candidates_offsets;         // [N + 1] dev_candidates_offsets (2 x SP words per event)
-    uint32_t* sp_scratch;                       // [S] sorted bank copies of events whose copies do not
-                                                //     fit the shared-memory blob (null: full scans)
-    unsigned sp_capacity;                       // S, allocated words of sp_scratch
-    const unsigned* sp_base;                    // [N] where the estimate kernel sorted each event's banks
-                                                //     in sp_scratch (null: this kernel sorts them)
+    const uint32_t* list_scratch;               // the estimate kernel's candidates: module_candidate_num[e]
+    const unsigned* list_base;                  // [N]  words from list_base[e] on (null: found again here)
+    const unsigned* module_candidate_num;       // [N]
     unsigned* status;
     unsigned smem_blob_bytes;
     unsigned smem_cluster_capacity;             // clusters staged in shared memory per event
