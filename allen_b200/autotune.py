@@ -25,9 +25,7 @@ SEARCH_VARIANTS = [(128, 1, 0), (128, 2, 0), (256, 1, 0), (256, 2, 0), (256, 4, 
                    (128, 0, 0), (256, 0, 0), (512, 0, 0), (64, 0, 1), (96, 0, 1), (128, 0, 1), (256, 0, 1)]
 SEARCH_CAPACITIES = [0, 1024, 2048, 2560, 3072, 4096]
 CLUSTER_CAPACITIES = [0, 1024, 2048, 2560, 3072]
-CLUSTER_BLOBS = [0, 16 * 1024, 24 * 1024, 32 * 1024, 40 * 1024]
 CLUSTER_THREADS = [256, 128]
-ESTIMATE_BLOBS = [0, 16 * 1024, 24 * 1024, 32 * 1024, 48 * 1024]
 # (persistent, events per claim): one CTA per event, or resident CTAs claiming events
 QUEUES = [(0, 1), (1, 1), (1, 2), (1, 4)]
 
@@ -72,8 +70,6 @@ def tune(chain, dev_slices, log=print, max_sweeps: int = 3) -> tuple[dict, float
         ("search_hit_capacity", SEARCH_CAPACITIES),
         ("cluster_stage_capacity", CLUSTER_CAPACITIES),
         ("cluster_threads", CLUSTER_THREADS),
-        ("cluster_blob_bytes", CLUSTER_BLOBS),
-        ("estimate_blob_bytes", ESTIMATE_BLOBS),
         ("queue", QUEUES),
     )
     # sweeps repeat until one changes nothing: the best search kernel depends on the staging

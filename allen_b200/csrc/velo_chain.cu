@@ -2,8 +2,10 @@
 // workspace, the launch sequence of the chain, CUDA-graph capture and the host-buffer path.
 //
 // Launch sequence for one slice of N events, on the caller's stream, no host sync:
-//   memset(bank index, status)
-//   estimate_kernel        [N CTAs]  velo_calculate_number_of_candidates + velo_estimate_input_size
+//   memset(bank index, status, counters)
+//   event_order_kernel               order of the events for persistent launches, bank index
+//   estimate_kernel        [N CTAs]  velo_calculate_number_of_candidates + velo_estimate_input_size,
+//                                    and the pixel sums of the clusters
 //   exclusive_scan_kernel  [2 jobs]  prefix_sum_offsets_velo_candidates, event estimate bases
 //   cluster_sort_kernel    [N CTAs]  velo_masked_clustering + velo_sort_by_phi
 //                                    (+ prefix_sum_offsets_estimated_input_size, per event)
@@ -253,7 +255,7 @@ struct VeloChain {
   size_t cap_track_hits = 0;
 
   // launch configuration (autotuned by allen_b200/autotune.py)
-  unsigned estimate_blob_bytes = 32 * 1024;
+  unsigned estimate_blob_bytes = 32 * 1024; // no effect: the kernels do not stage raw events
   unsigned cluster_blob_bytes = 16 * 1024;
   unsigned cluster_stage_capacity = 3072;
   unsigned search_hit_capacity = 3072;
@@ -278,8 +280,9 @@ struct VeloChain {
     event_track_hits, event_track_hit_base, offsets_all, track_hit_number, offsets_hit_number;
   DeviceBuffer<char> sorted, staging, track_hits, hit_scratch;
   DeviceBuffer<uint64_t> ring_scratch; // search_ring_global: one ring of 2048 entries per resident search CTA
-  DeviceBuffer<uint32_t> list_scratch; // candidates the estimate kernel leaves to the clustering kernel
-  DeviceBuffer<unsigned> list_base, list_alloc; // each event's place in list_scratch, the allocation counter
+  DeviceBuffer<uint32_t> list_scratch; // items the estimate kernel leaves to the clustering kernel
+  DeviceBuffer<unsigned> list_alloc;   // its allocation counter
+  DeviceBuffer<uint4> lists;           // each event's part of it
   DeviceBuffer<velo::TrackHits> tracks;
   DeviceBuffer<velo::TrackletHits> three_hit, three_out;
   DeviceBuffer<uint8_t> hit_used, accepted;
@@ -390,8 +393,8 @@ namespace {
     f(c->event_track_hit_base, n + 1, scratch_buffer);
     f(c->staging, 24 * T, scratch_buffer);
     f(c->hit_scratch, 16 * T, scratch_buffer);
-    f(c->list_scratch, b.super_pixels + 64, scratch_buffer);
-    f(c->list_base, n, scratch_buffer);
+    f(c->list_scratch, 2 * b.super_pixels + 64, scratch_buffer);
+    f(c->lists, n, scratch_buffer);
     f(c->list_alloc, 1, scratch_buffer);
     f(c->tracks, tracks, scratch_buffer);
     f(c->three_hit, tracks, scratch_buffer);
@@ -518,7 +521,10 @@ namespace {
     auto grid = [&](unsigned resident) { return persistent ? std::min(n, std::max(resident, 1u)) : n; };
     if (persistent) {
       VELO_CUDA(cudaMemsetAsync(c->queue_next.p, 0, 3 * sizeof(unsigned), stream));
-      event_order_kernel<<<1, scan_threads, 0, stream>>>(in, c->event_order.p);
+    }
+    if (persistent || !c->retina) {
+      event_order_kernel<<<event_order_grid(n, !c->retina), scan_threads, 0, stream>>>(
+        in, persistent ? c->event_order.p : nullptr, bank_index_stride(n), c->bank_index_key.p);
       VELO_CUDA(cudaGetLastError());
     }
     VELO_CUDA(mark());
@@ -565,16 +571,14 @@ namespace {
       ep.module_candidate_num = c->candidate_num.p;
       ep.event_estimate = c->event_estimate.p;
       ep.bank_index_key = c->bank_index_key.p;
-      ep.designated_stride = (n + 255) / 256;
       ep.status = c->status.p;
-      ep.smem_blob_bytes = c->estimate_blob_bytes;
       ep.list_scratch = c->list_scratch.p;
       ep.list_capacity = static_cast<unsigned>(c->list_scratch.n);
       ep.list_alloc = c->list_alloc.p;
-      ep.list_base = c->list_base.p;
+      ep.lists = c->lists.p;
       ep.queue = queue(0);
       VELO_CUDA(cudaMemsetAsync(c->list_alloc.p, 0, sizeof(unsigned), stream));
-      estimate_kernel<<<grid(c->resident_estimate), decode_threads, c->estimate_blob_bytes, stream>>>(ep);
+      estimate_kernel<<<grid(c->resident_estimate), decode_threads, 0, stream>>>(ep);
       VELO_CUDA(cudaGetLastError());
       VELO_CUDA(mark());
 
@@ -597,13 +601,11 @@ namespace {
       cp.sorted_container = c->sorted.p;
       cp.staging = c->staging.p;
       cp.list_scratch = c->list_scratch.p;
-      cp.list_base = c->list_base.p;
-      cp.module_candidate_num = c->candidate_num.p;
+      cp.lists = c->lists.p;
       cp.status = c->status.p;
-      cp.smem_blob_bytes = c->cluster_blob_bytes;
-      cp.smem_cluster_capacity = c->cluster_stage_capacity;
+      cp.smem_cluster_capacity = std::max(c->cluster_stage_capacity, min_cluster_stage);
       cp.cluster_capacity = static_cast<unsigned>(c->cap_clusters);
-      const unsigned cluster_smem = cluster_sort_blob_offset(c->cluster_stage_capacity) + c->cluster_blob_bytes;
+      const unsigned cluster_smem = cluster_sort_smem(std::max(c->cluster_stage_capacity, min_cluster_stage));
       cp.queue = queue(1);
       if (c->cluster_threads == 128)
         cluster_sort_kernel<128><<<grid(c->resident_cluster), 128, cluster_smem, stream>>>(cp);
@@ -756,9 +758,8 @@ namespace {
   VeloStatus configure_kernels(VeloChain* c)
   {
     using namespace velo;
-    const int cluster_smem = int(cluster_sort_blob_offset(c->cluster_stage_capacity) + c->cluster_blob_bytes);
+    const int cluster_smem = int(cluster_sort_smem(std::max(c->cluster_stage_capacity, min_cluster_stage)));
     const int search_smem = int(c->search_hit_capacity * search_hit_bytes);
-    VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(estimate_kernel), int(c->estimate_blob_bytes)));
     VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(cluster_sort_kernel<128>), cluster_smem));
     VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(cluster_sort_kernel<256>), cluster_smem));
     for (const auto& v : search_variants)
@@ -770,7 +771,7 @@ namespace {
     // CTAs of each kernel resident on the device at once: the grid of a persistent launch
     int sms = 0, per_sm = 0;
     VELO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, estimate_kernel, decode_threads, c->estimate_blob_bytes));
+    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, estimate_kernel, decode_threads, 0));
     c->resident_estimate = unsigned(std::max(per_sm, 1) * sms);
     VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kalman_filter_kernel, kalman_threads, 0));
     c->resident_kalman = unsigned(std::max(per_sm, 1) * sms);
@@ -1055,7 +1056,7 @@ VeloStatus velo_chain_configure(VeloChain* c, const VeloLaunchConfig* cfg)
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
   const unsigned search_static = 32 * 1024; // upper bound of the kernel's static shared memory
-  const unsigned cluster_dyn = velo::cluster_sort_blob_offset(cfg->cluster_stage_capacity) + cfg->cluster_blob_bytes;
+  const unsigned cluster_dyn = velo::cluster_sort_smem(cfg->cluster_stage_capacity) + cfg->cluster_blob_bytes;
   if (cfg->search_hit_capacity * velo::search_hit_bytes + search_static > unsigned(optin) ||
       cluster_dyn + 16 * 1024 > unsigned(optin) || cfg->estimate_blob_bytes + 16 * 1024 > unsigned(optin) ||
       cfg->search_hit_capacity > 65536 || cfg->cluster_stage_capacity > 65535 || (cfg->cluster_blob_bytes & 15) ||

@@ -37,7 +37,7 @@ namespace velo {
     err_track_capacity = 1u << 1,    // an event produced more tracks than its container slice
     err_ttf_overflow = 1u << 2,      // more than 2048 tracks in flight in one event
     err_bad_sensor = 1u << 3,        // a candidate names a sensor outside the geometry
-    err_bulk_copy_timeout = 1u << 4, // a bulk copy into shared memory did not complete in time
+    err_bulk_copy_timeout = 1u << 4, // (no kernel raises it any more)
     err_output_capacity = 1u << 5,   // consolidated output larger than the reserved buffer
     err_input_capacity = 1u << 6,    // slice larger than the reserved workspace
     err_hits_per_event = 1u << 7,    // more than 65535 estimated hits in one event (u16 indices)

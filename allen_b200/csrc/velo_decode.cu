@@ -2,14 +2,14 @@
 // (velo_calculate_number_of_candidates + velo_estimate_input_size), masked clustering,
 // phi and the sort by phi (velo_masked_clustering + velo_sort_by_phi), one event per CTA.
 //
-// A CTA reads its event's raw blob (bank offsets + SP words) through L1/L2, or stages it
-// into shared memory with one bulk copy through the TMA engine (cp.async.bulk, 16-byte
-// aligned span, the ragged tail by plain loads) when the launch configuration gives it room.
+// The estimate kernel reads an event's super pixels once into shared memory, one thread per
+// super pixel over the flattened bank list, sizes the event, and leaves an item per cluster to
+// make: the isolated super pixels, and the pixel sums of the clusters that the candidates among
+// the others grow into.  The clustering kernel turns the items into hits with every lane busy
+// and sorts them; it needs neither the raw words nor a bank table.
 // The neighbour scans of the reference (EstimateInputSize.cu:111-141,
 // MaskedVeloClustering.cu:361-402) test the address of every super pixel of a bank against one
-// range (four instructions each) and look closer at the few inside it; the estimate kernel
-// leaves the candidates it finds to the clustering kernel, so each is found once.
-// Work is spread one thread per super pixel over the flattened bank list.
+// range (four instructions each) and look closer at the few inside it.
 //
 // The sorted container is independent of the order in which clusters are produced
 // (rank by (phi, id), SortByPhi.cu:104-122), so clusters are appended to their module
@@ -23,292 +23,148 @@ namespace velo {
   constexpr unsigned estimate_words = 3584; // SPs of an event that the estimate kernel holds in shared memory
 
   // ------------------------------------------------------------------------------------
-  // Bulk copy (TMA engine) into shared memory, completion tracked by an mbarrier.
-  // ------------------------------------------------------------------------------------
-  __device__ __forceinline__ uint32_t smem_u32(const void* p)
-  {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-  }
-
-  __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count)
-  {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-
-  __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes)
-  {
-    uint64_t state;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 %0, [%1], %2;"
-                 : "=l"(state)
-                 : "r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-    (void) state;
-  }
-
-  __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar)
-  {
-    asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src),
-      "r"(bytes),
-      "r"(smem_u32(bar))
-      : "memory");
-  }
-
-  __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned phase)
-  {
-    uint32_t done;
-    asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(phase)
-      : "memory");
-    return done != 0;
-  }
-
-  constexpr unsigned bulk_wait_limit = 1u << 22; // try_wait rounds before giving up
-
-  // Stages the event blob into `smem_blob` (16-byte aligned) when it fits; returns the
-  // address of the event's first word (shared or global) and its length in words.
-  // Ends with a __syncthreads().  `bar` must have been initialised with count 1; bar_phase
-  // (the same in every thread) is the parity of its current phase.
-  __device__ const uint32_t* stage_event(
-    const RawInput& in,
-    unsigned ev,
-    unsigned char* smem_blob,
-    unsigned smem_blob_bytes,
-    uint64_t* bar,
-    unsigned& bar_phase,
-    unsigned* status,
-    unsigned& n_words,
-    unsigned& staged_bytes)
-  {
-    staged_bytes = 0;
-    if (in.mep_layout) {
-      // the event's banks are scattered over the MEP: read in place
-      n_words = 0xFFFFFFFFu;
-      __syncthreads();
-      return reinterpret_cast<const uint32_t*>(in.raw);
-    }
-    const unsigned begin = in.offsets[ev];
-    const unsigned end = in.offsets[ev + 1];
-    n_words = (end - begin) / 4;
-    const char* src = in.raw + begin;
-    const uintptr_t s = reinterpret_cast<uintptr_t>(src);
-    const uintptr_t e = s + (end - begin);
-    const uintptr_t s_al = s & ~uintptr_t(15);
-    const uintptr_t e_al = e & ~uintptr_t(15);
-    const unsigned need = static_cast<unsigned>(((e + 15) & ~uintptr_t(15)) - s_al);
-    const bool base_aligned = (reinterpret_cast<uintptr_t>(in.raw) & 15u) == 0;
-    if (!base_aligned || need > smem_blob_bytes) {
-      __syncthreads();
-      return reinterpret_cast<const uint32_t*>(src);
-    }
-    const unsigned bulk = e_al > s_al ? static_cast<unsigned>(e_al - s_al) : 0u;
-    if (threadIdx.x == 0 && bulk > 0) {
-      mbar_expect_tx(bar, bulk);
-      bulk_copy_g2s(smem_blob, reinterpret_cast<const void*>(s_al), bulk, bar);
-    }
-    // ragged tail (whole 32-bit words) by plain loads
-    const uintptr_t tail = e_al > s ? e_al : s;
-    for (uintptr_t a = tail + 4 * threadIdx.x; a < e; a += 4 * blockDim.x) {
-      *reinterpret_cast<uint32_t*>(smem_blob + (a - s_al)) = *reinterpret_cast<const uint32_t*>(a);
-    }
-    bool ok = true;
-    if (bulk > 0) {
-      unsigned rounds = 0;
-      while (!mbar_try_wait(bar, bar_phase)) {
-        if (++rounds > bulk_wait_limit) {
-          ok = false;
-          break;
-        }
-      }
-      bar_phase ^= 1u; // each completed copy advances the barrier by one phase
-    }
-    __syncthreads();
-    if (!ok) {
-      if (threadIdx.x == 0) set_error(status, err_bulk_copy_timeout);
-      return reinterpret_cast<const uint32_t*>(src);
-    }
-    staged_bytes = need;
-    return reinterpret_cast<const uint32_t*>(smem_blob + (s - s_al));
-  }
-
-  // ------------------------------------------------------------------------------------
   // Bank table of one event (ClusteringDefinitions.cuh:61-144)
   // ------------------------------------------------------------------------------------
-  struct BankTable {
-    unsigned n_banks;
-    unsigned total_sp;
-    unsigned count_total;
-    unsigned words_off[max_banks]; // first SP word of the bank, in words from the event start
-    unsigned n_sp[max_banks];      // SP words of the bank (any bank type)
-    unsigned flat[max_banks + 1];  // exclusive scan of n_sp over VP/Velo banks
-    unsigned source_id[max_banks];
-    uint8_t velo[max_banks];
-    // hint[k]: the bank holding flat SP k * 32 (entries up to total_sp / 32), where bank_of()
-    // starts a short forward scan
-    uint16_t hint[bank_hints];
-  };
-
   __device__ __forceinline__ unsigned bank_module_pair(unsigned source_id, int version)
   {
     return (version == 2 || version == 3) ? (source_id & 0x1FFu) / 8 : ((source_id & 0x1FFu) << 1) / 8;
   }
 
-  // MEP layout: the same table, with word offsets relative to the start of `raw` (the words
-  // pointer stage_event returns).  A fragment must start on a 4-byte boundary; its word count
-  // is clamped to the bank size.  Ends with a __syncthreads().
-  __device__ void parse_banks_mep(const RawInput& in, unsigned ev, BankTable& bt, unsigned* warp_sums, unsigned* status)
+  // The words of an event: its own (Allen layout), or all of a MEP's, whose banks are scattered.
+  struct EventWords {
+    const uint32_t* w;
+    unsigned n;           // words of the event (MEP: no bound)
+    unsigned n_banks_raw; // as the event states it
+    unsigned n_banks;     // at most max_banks
+  };
+
+  __device__ __forceinline__ EventWords event_words(const RawInput& in, unsigned ev)
+  {
+    EventWords r;
+    if (in.mep_layout) {
+      r.w = reinterpret_cast<const uint32_t*>(in.raw);
+      r.n = 0xFFFFFFFFu;
+      r.n_banks_raw = mep_n_banks(in);
+    }
+    else {
+      const unsigned begin = in.offsets[ev];
+      r.w = reinterpret_cast<const uint32_t*>(in.raw + begin);
+      r.n = (in.offsets[ev + 1] - begin) / 4;
+      r.n_banks_raw = r.n > 0 ? r.w[0] : 0u;
+    }
+    r.n_banks = min(r.n_banks_raw, max_banks);
+    return r;
+  }
+
+  struct Bank {
+    unsigned first;     // first SP word
+    unsigned n_sp;      // SP words (any bank type), clamped to the event or the fragment
+    unsigned stated;    // SP words as the bank states them
+    unsigned source_id;
+    bool velo;
+    bool bad;           // the stated words do not fit
+  };
+
+  // Bank b < n_banks of an event.  A MEP fragment must start on a 4-byte boundary; its word
+  // count is clamped to the bank size.
+  __device__ __forceinline__ Bank event_bank(const RawInput& in, unsigned ev, const EventWords& e, unsigned b)
   {
     const bool v23 = in.bank_version == 2 || in.bank_version == 3;
-    const unsigned n_banks_raw = mep_n_banks(in);
-    const unsigned n_banks = n_banks_raw < max_banks ? n_banks_raw : max_banks;
-    if (n_banks_raw > max_banks && threadIdx.x == 0) set_error(status, err_input_capacity);
-    const uint32_t* raw32 = reinterpret_cast<const uint32_t*>(in.raw);
-    unsigned carry = 0, count = 0;
-    for (unsigned base = 0; base < n_banks; base += blockDim.x) {
-      const unsigned b = base + threadIdx.x;
-      unsigned nsp_flat = 0;
-      if (b < n_banks) {
-        const unsigned frag = mep_fragment_offset(in, ev, b);
-        const unsigned size = mep_bank_size(in, ev, b);
-        const unsigned type = mep_bank_type(in, ev, b);
-        const bool velo_bank = type == bank_type_vp || type == bank_type_velo;
-        unsigned nsp = 0, first = 0;
-        if (frag & 3u) {
-          set_error(status, err_input_capacity);
-        }
-        else if (v23) {
-          nsp = size >= 4 ? raw32[frag / 4] : 0u;
-          first = frag / 4 + 1;
-          if (velo_bank) count += nsp;
-          if (nsp > (size >= 4 ? size / 4 - 1 : 0u)) {
-            set_error(status, err_input_capacity);
-            nsp = size >= 4 ? size / 4 - 1 : 0u;
-          }
-        }
-        else {
-          nsp = size / 4u;
-          first = frag / 4;
-          if (velo_bank) count += nsp;
-        }
-        bt.words_off[b] = first;
-        bt.n_sp[b] = nsp;
-        bt.source_id[b] = mep_source_id(in, b);
-        bt.velo[b] = velo_bank;
-        nsp_flat = velo_bank ? nsp : 0u;
+    Bank r;
+    r.bad = false;
+    if (in.mep_layout) {
+      const unsigned frag = mep_fragment_offset(in, ev, b);
+      const unsigned size = mep_bank_size(in, ev, b);
+      const unsigned type = mep_bank_type(in, ev, b);
+      r.velo = type == bank_type_vp || type == bank_type_velo;
+      r.source_id = mep_source_id(in, b);
+      r.stated = r.n_sp = r.first = 0;
+      if (frag & 3u) {
+        r.bad = true;
       }
-      unsigned total;
-      const unsigned excl = block_exclusive_scan(nsp_flat, warp_sums, &total);
-      if (b < n_banks) bt.flat[b] = carry + excl;
-      carry += total;
+      else if (v23) {
+        r.stated = size >= 4 ? e.w[frag / 4] : 0u;
+        r.first = frag / 4 + 1;
+        const unsigned room = size >= 4 ? size / 4 - 1 : 0u;
+        r.bad = r.stated > room;
+        r.n_sp = min(r.stated, room);
+      }
+      else {
+        r.stated = r.n_sp = size / 4u;
+        r.first = frag / 4;
+      }
+      return r;
     }
-    unsigned total_count;
-    block_exclusive_scan(count, warp_sums, &total_count);
-    if (threadIdx.x == 0) {
-      bt.n_banks = n_banks;
-      bt.total_sp = carry;
-      bt.flat[n_banks] = carry;
-      bt.count_total = total_count;
+    const unsigned off = (1 + b < e.n) ? e.w[1 + b] : 0u;
+    const unsigned w = 2 + e.n_banks_raw + off / 4;
+    const unsigned type = bank_types(in, ev)[b];
+    r.velo = type == bank_type_vp || type == bank_type_velo;
+    r.source_id = w < e.n ? e.w[w] : 0u;
+    if (v23) {
+      r.stated = (w + 1 < e.n) ? e.w[w + 1] : 0u;
+      r.first = w + 2;
     }
-    __syncthreads();
+    else {
+      r.stated = bank_sizes(in, ev)[b] / 4u;
+      r.first = w + 1;
+    }
+    r.n_sp = r.stated;
+    if (r.first > e.n) r.first = e.n;
+    if (r.first + r.n_sp > e.n || r.first + r.n_sp < r.first) {
+      r.bad = true;
+      r.n_sp = e.n - r.first;
+    }
+    return r;
   }
+
+  struct BankTable {
+    unsigned n_banks;
+    unsigned total_sp;
+    unsigned count_total;          // SP words of VP/Velo banks as stated (reference: raw_bank.count or size / 4)
+    unsigned words_off[max_banks]; // first SP word of the bank, in words from the event start
+    unsigned flat[max_banks + 1];  // exclusive scan of the SP words over VP/Velo banks
+    unsigned source_id[max_banks];
+    // hint[k]: the bank holding flat SP k * 32 (entries up to total_sp / 32), where the searches
+    // for an SP's bank start
+    uint16_t hint[bank_hints];
+  };
 
   // Fills the table; ends with a __syncthreads().
   __device__ void parse_banks(
-    const RawInput& in,
-    unsigned ev,
-    const uint32_t* words,
-    unsigned n_words,
-    BankTable& bt,
-    unsigned* warp_sums,
-    unsigned* status)
+    const RawInput& in, unsigned ev, const EventWords& e, BankTable& bt, unsigned* warp_sums, unsigned* status)
   {
-    const bool v23 = in.bank_version == 2 || in.bank_version == 3;
-    if (in.mep_layout) {
-      parse_banks_mep(in, ev, bt, warp_sums, status);
-      return;
+    if (threadIdx.x == 0) {
+      bt.count_total = 0;
+      if (e.n_banks_raw > max_banks) set_error(status, err_input_capacity);
     }
-    const unsigned n_banks_raw = n_words > 0 ? words[0] : 0u;
-    const unsigned n_banks = n_banks_raw < max_banks ? n_banks_raw : max_banks;
-    if (n_banks_raw > max_banks && threadIdx.x == 0) set_error(status, err_input_capacity);
-    const uint16_t* sizes = bank_sizes(in, ev);
-    const uint8_t* types = bank_types(in, ev);
     unsigned carry = 0, count = 0;
-    for (unsigned base = 0; base < n_banks; base += blockDim.x) {
+    for (unsigned base = 0; base < e.n_banks; base += blockDim.x) {
       const unsigned b = base + threadIdx.x;
       unsigned nsp_flat = 0;
-      if (b < n_banks) {
-        const unsigned off = (1 + b < n_words) ? words[1 + b] : 0u;
-        const unsigned w = 2 + n_banks_raw + off / 4;
-        const unsigned type = types[b];
-        const bool velo_bank = type == bank_type_vp || type == bank_type_velo;
-        const unsigned src = w < n_words ? words[w] : 0u;
-        unsigned nsp, first;
-        if (v23) {
-          nsp = (w + 1 < n_words) ? words[w + 1] : 0u;
-          first = w + 2;
+      if (b < e.n_banks) {
+        const Bank bank = event_bank(in, ev, e, b);
+        if (bank.bad) set_error(status, err_input_capacity);
+        if (bank.velo) {
+          count += bank.stated;
+          nsp_flat = bank.n_sp;
         }
-        else {
-          nsp = sizes[b] / 4u;
-          first = w + 1;
-        }
-        if (velo_bank) count += nsp;
-        if (first > n_words) first = n_words;
-        if (first + nsp > n_words || first + nsp < first) {
-          set_error(status, err_input_capacity);
-          nsp = n_words - first;
-        }
-        bt.words_off[b] = first;
-        bt.n_sp[b] = nsp;
-        bt.source_id[b] = src;
-        bt.velo[b] = velo_bank;
-        nsp_flat = velo_bank ? nsp : 0u;
+        bt.words_off[b] = bank.first;
+        bt.source_id[b] = bank.source_id;
       }
       unsigned total;
       const unsigned excl = block_exclusive_scan(nsp_flat, warp_sums, &total);
-      if (b < n_banks) bt.flat[b] = carry + excl;
+      if (b < e.n_banks) bt.flat[b] = carry + excl;
       carry += total;
     }
-    // count of SP words of VP/Velo banks, unclamped (reference: raw_bank.count or size / 4)
-    unsigned total_count;
-    block_exclusive_scan(count, warp_sums, &total_count);
+    count = __reduce_add_sync(0xFFFFFFFFu, count);
+    if ((threadIdx.x & 31u) == 0 && count) atomicAdd(&bt.count_total, count);
     if (threadIdx.x == 0) {
-      bt.n_banks = n_banks;
+      bt.n_banks = e.n_banks;
       bt.total_sp = carry;
-      bt.flat[n_banks] = carry;
-      bt.count_total = total_count;
+      bt.flat[e.n_banks] = carry;
     }
     __syncthreads();
-  }
-
-  // atomicAdd(counter, 1) from the converged lanes of the warp, one atomic per counter (the
-  // lanes that add to the same counter pass the same key): returns this lane's old value, the
-  // lanes of a key taking consecutive values in lane order.
-  __device__ __forceinline__ unsigned warp_aggregated_inc(unsigned* counter, unsigned key)
-  {
-    const unsigned peers = __match_any_sync(__activemask(), key);
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned leader = __ffs(peers) - 1;
-    unsigned base = 0;
-    if (lane == leader) base = atomicAdd(counter, static_cast<unsigned>(__popc(peers)));
-    return __shfl_sync(peers, base, leader) + __popc(peers & ((1u << lane) - 1u));
-  }
-
-  // atomicAdd(counter, v) from the converged lanes of the warp, one atomic per counter.
-  __device__ __forceinline__ void warp_aggregated_add(unsigned* counter, unsigned key, unsigned v)
-  {
-    const unsigned peers = __match_any_sync(__activemask(), key);
-    const unsigned sum = __reduce_add_sync(peers, v);
-    if ((threadIdx.x & 31u) == static_cast<unsigned>(__ffs(peers) - 1) && sum) atomicAdd(counter, sum);
-  }
-
-  // The hint table of a parsed bank table; ends with a __syncthreads().
-  __device__ __forceinline__ void index_banks(BankTable& bt)
-  {
-    for (unsigned b = threadIdx.x; b < bt.n_banks; b += blockDim.x) {
+    for (unsigned b = threadIdx.x; b < e.n_banks; b += blockDim.x) {
       const unsigned hi = bt.flat[b + 1];
       for (unsigned k = (bt.flat[b] + 31) / 32; k < bank_hints && k * 32 < hi; ++k)
         bt.hint[k] = static_cast<uint16_t>(b);
@@ -316,15 +172,37 @@ namespace velo {
     __syncthreads();
   }
 
+  // Adds each lane's v (0, 1 or 2) to its counter, from converged lanes: one atomic when all
+  // lanes name the same counter.
+  __device__ __forceinline__ void add_to_counter(unsigned* counters, unsigned key, unsigned v)
+  {
+    const unsigned lanes = __activemask(), leader = __ffs(lanes) - 1;
+    if (__all_sync(lanes, key == __shfl_sync(lanes, key, leader))) {
+      const unsigned sum = __popc(__ballot_sync(lanes, v > 0)) + __popc(__ballot_sync(lanes, v > 1));
+      if ((threadIdx.x & 31u) == leader && sum) atomicAdd(counters + key, sum);
+    }
+    else if (v) {
+      atomicAdd(counters + key, v);
+    }
+  }
+
+  // Places for the converged lanes' items (v of 0, 1 or 2 each) behind *counter: one atomic per
+  // warp.  Returns the place of a lane's first item; its second one lies at `second`.
+  __device__ __forceinline__ unsigned append_items(unsigned* counter, unsigned v, unsigned& second)
+  {
+    const unsigned lanes = __activemask(), leader = __ffs(lanes) - 1, lane = threadIdx.x & 31u;
+    const unsigned one = __ballot_sync(lanes, v > 0), two = __ballot_sync(lanes, v > 1);
+    unsigned at = 0;
+    if (lane == leader) at = atomicAdd(counter, static_cast<unsigned>(__popc(one) + __popc(two)));
+    at = __shfl_sync(lanes, at, leader);
+    const unsigned below = (1u << lane) - 1u;
+    second = at + __popc(one) + __popc(two & below);
+    return at + __popc(one & below);
+  }
+
   __device__ __forceinline__ unsigned bank_of(const BankTable& bt, unsigned f)
   {
     // last bank b with flat[b] <= f < total_sp (banks with no SP share their start with the next)
-    if (f / 32 < bank_hints) {
-      unsigned b = bt.hint[f / 32];
-      while (b + 1 < bt.n_banks && bt.flat[b + 1] <= f)
-        ++b;
-      return b;
-    }
     unsigned lo = 0, hi = bt.n_banks;
     while (hi - lo > 1) {
       const unsigned mid = (lo + hi) / 2;
@@ -334,16 +212,33 @@ namespace velo {
     return lo;
   }
 
+  // bank_of() of the 32 consecutive SPs of a warp (f of lane 0 a multiple of 32, every lane of
+  // the warp calls it): the lanes hold the starts of the banks behind the hint and bisect them
+  // by shuffles.  Beyond the last SP the result is some bank.
+  __device__ __forceinline__ unsigned bank_of_warp(const BankTable& bt, unsigned f)
+  {
+    const unsigned k = f / 32;
+    const bool hinted = k < bank_hints && (f & ~31u) < bt.total_sp;
+    const unsigned b0 = hinted ? bt.hint[k] : 0u;
+    const unsigned next = b0 + 1 + (threadIdx.x & 31u);
+    const unsigned start = next < bt.n_banks ? bt.flat[next] : 0xFFFFFFFFu;
+    unsigned n = 0;
+#pragma unroll
+    for (unsigned step = 16; step >= 1; step /= 2)
+      if (__shfl_sync(0xFFFFFFFFu, start, n + step - 1) <= f) n += step;
+    if (!hinted || n == 31) return f < bt.total_sp ? bank_of(bt, f) : 0u;
+    return b0 + n;
+  }
+
   // ------------------------------------------------------------------------------------
   // Neighbour scans.  The reference visits every SP of the bank for every SP
   // (EstimateInputSize.cu:111-141) and every candidate (MaskedVeloClustering.cu:361-402).  The
   // SPs that can matter lie in one short range of addresses (column, then row), so the scan
   // only notes which SPs of the bank are in the range, a bit each, and the caller looks at
   // those: about one of the 12 to 24 SPs a bank holds, and a lane that has none does not wait
-  // for the others at every SP.  Against key-sorted bank copies searched by bisection (the sort
-  // alone compared every pair of a bank's SPs), with the candidates handed over: estimate
-  // 0.94 -> 0.79 ms and clustering 1.85 -> 1.31 ms for 16000 events of 2540 SPs, 0.77 -> 0.40 and
-  // 0.98 -> 0.66 ms for 2000 of 8200 SPs (version 4, 78 SPs per bank).
+  // for the others at every SP.  (Against key-sorted bank copies searched by bisection, whose sort
+  // compares every pair of a bank's SPs: estimate and clustering together 2.79 -> 2.10 ms for
+  // 16000 events of 2540 SPs, 1.75 -> 1.06 ms for 2000 of 8200 SPs, version 4, 78 SPs per bank.)
   // ------------------------------------------------------------------------------------
   // visit(w) for the SPs among bank_words[0, n) with lo <= ((w >> 8) & key_mask) <= lo + span, in order.
   template<typename Visit>
@@ -371,39 +266,25 @@ namespace velo {
   // no-neighbour bit instead of the other's (line 113), which is always 0 here.
   // Returns up to two candidate pixel codes: bit 8 set = present, bits 0..2 = pixel.
   // ------------------------------------------------------------------------------------
-  __device__ __forceinline__ void
-  add_neighbour_pixels(uint32_t& pixels, uint32_t ow, uint32_t sp_row, uint32_t sp_col)
-  {
-    const uint32_t oaddr = (ow & 0x007FFF00u) >> 8;
-    const uint32_t orow = oaddr & 0x3Fu;
-    const uint32_t ocol = oaddr >> 6;
-    const uint32_t osp = ow & 0xFFu;
-    const bool col_same = ocol == sp_col;
-    const bool col_right = ocol == sp_col + 1;
-    if (!(col_same || col_right)) return;
-    if (orow == sp_row + 1) {
-      if (col_same) pixels |= (((osp & 0x01u) | ((osp & 0x10u) << 2)) << 4);
-      else pixels |= ((osp & 0x01u) << 16);
-    }
-    else if (orow == sp_row) {
-      if (col_right) pixels |= ((osp & 0x0Fu) << 12);
-    }
-    else if (orow == sp_row - 1) {
-      if (col_right) pixels |= ((osp & 0x08u) << 8);
-      else pixels |= ((osp & 0x80u) >> 2);
-    }
-  }
-
   // Neighbours of either sensor of a version 4 bank count (the reference compares bits 22:8 only).
   __device__ __forceinline__ uint32_t sp_candidates(uint32_t sp_word, const uint32_t* bank_words, unsigned n_sp)
   {
     const uint32_t sp_addr = (sp_word & 0x007FFF00u) >> 8;
     const uint32_t sp = sp_word & 0xFFu;
     uint32_t pixels = (sp & 0x0Fu) | ((sp & 0xF0u) << 2);
-    const uint32_t sp_row = sp_addr & 0x3Fu;
-    const uint32_t sp_col = sp_addr >> 6;
-    // same column, one row below, to next column, one row above (the SP itself adds nothing)
-    scan_keys(bank_words, n_sp, sp_addr - 1, 66, 0x7FFFu, [&](uint32_t ow) { add_neighbour_pixels(pixels, ow, sp_row, sp_col); });
+    const uint32_t row = sp_addr & 0x3Fu;
+    // Addresses from one row below in the same column to one row above in the next (the SP itself
+    // adds nothing); a row beyond the column's ends is another column's.
+    scan_keys(bank_words, n_sp, sp_addr - 1, 66, 0x7FFFu, [&](uint32_t ow) {
+      const uint32_t ahead = ((ow & 0x007FFF00u) >> 8) - sp_addr;
+      const bool above = row < 63 && (ahead == 1 || ahead == 65), below = row > 0 && (ahead == ~0u || ahead == 63);
+      const bool next = ahead > 62 && ahead <= 65;
+      uint32_t add = 0;
+      if (above) add = next ? (ow & 0x01u) << 16 : ((ow & 0x01u) << 4) | ((ow & 0x10u) << 6);
+      if (below) add = next ? (ow & 0x08u) << 8 : (ow & 0x80u) >> 2;
+      if (ahead == 64) add = (ow & 0x0Fu) << 12;
+      pixels |= add;
+    });
     const uint32_t inside = pixels & 0x3CFu;
     const uint32_t mask = (inside << 1) | (inside << 5) | (inside << 6) | (inside << 7);
     const uint32_t working = mask & (~pixels);
@@ -423,161 +304,6 @@ namespace velo {
     const bool pattern_0 = (sp & 0x88u) && !(sp & 0x44u) && (sp & 0x33u);
     const bool pattern_1 = (sp & 0xCCu) && !(sp & 0x22u) && (sp & 0x11u);
     return pattern_0 || pattern_1;
-  }
-
-  constexpr unsigned estimate_queue = 1024; // SPs per chunk of the estimate (and queue entries)
-  static_assert(estimate_queue % decode_threads == 0, "every lane takes the same number of SPs per chunk");
-
-  // ------------------------------------------------------------------------------------
-  // estimate_kernel: dev_number_of_candidates, dev_velo_bank_index (as a max-reduced
-  // key), dev_estimated_input_size and dev_module_candidate_num.
-  // ------------------------------------------------------------------------------------
-  __device__ __forceinline__ void estimate_event(const EstimateParams& p, unsigned e, uint64_t* bar, unsigned& bar_phase)
-  {
-    extern __shared__ __align__(128) unsigned char dsmem[];
-    __shared__ BankTable bt;
-    __shared__ unsigned est_mp[n_module_pairs];
-    __shared__ unsigned cand_count;
-    __shared__ unsigned warp_sums[33];
-    __shared__ uint16_t queue[estimate_queue];
-    __shared__ unsigned queue_count[2];
-    __shared__ unsigned list_at;
-    __shared__ uint32_t held[estimate_words]; // the event's SPs in bank order, when they fit
-
-    const unsigned ev = e + p.in.event_start;
-    const bool v23 = p.in.bank_version == 2 || p.in.bank_version == 3;
-    if (threadIdx.x < n_module_pairs) est_mp[threadIdx.x] = 0;
-    if (threadIdx.x == 0) cand_count = 0;
-    if (threadIdx.x < 2) queue_count[threadIdx.x] = 0;
-    __syncthreads();
-
-    unsigned n_words, staged;
-    const uint32_t* words = stage_event(p.in, ev, dsmem, p.smem_blob_bytes, bar, bar_phase, p.status, n_words, staged);
-    parse_banks(p.in, ev, words, n_words, bt, warp_sums, p.status);
-    index_banks(bt);
-    (void) staged;
-    const bool in_smem = bt.total_sp <= estimate_words;
-    if (in_smem) {
-      for (unsigned f = threadIdx.x; f < bt.total_sp; f += blockDim.x) {
-        const unsigned b = bank_of(bt, f);
-        held[f] = words[bt.words_off[b] + f - bt.flat[b]];
-      }
-    }
-    // Room for the candidates this event hands to the clustering kernel, a word per SP (two
-    // clusters from one SP are rare); events that find none, or need more, hand over nothing.
-    if (threadIdx.x == 0) {
-      list_at = no_candidate_list;
-      if (p.list_scratch != nullptr) {
-        const unsigned at = atomicAdd(p.list_alloc, bt.total_sp);
-        if (at <= p.list_capacity && bt.total_sp <= p.list_capacity - at) list_at = at;
-      }
-    }
-    __syncthreads();
-    uint32_t* list = list_at != no_candidate_list ? p.list_scratch + list_at : nullptr;
-
-    // velo_calculate_number_of_candidates: block 0 of the reference's launch (grid of
-    // ceil(N / 256) blocks, one thread per event) handles events 0, stride, 2 stride, ...
-    // and the last of them to write an entry wins.
-    if (p.designated_stride > 0 && e % p.designated_stride == 0) {
-      const unsigned long long key_hi = static_cast<unsigned long long>(e) << 32;
-      for (unsigned b = threadIdx.x; b < bt.n_banks; b += blockDim.x) {
-        const unsigned src = bt.source_id[b] & 0x1FFu;
-        if (p.in.bank_version > 3) {
-          if ((src << 1) < n_sensors) atomicMax(p.bank_index_key + (src << 1), key_hi | b);
-          if (((src << 1) | 1u) < n_sensors) atomicMax(p.bank_index_key + ((src << 1) | 1u), key_hi | b);
-        }
-        else if (src < n_sensors) {
-          atomicMax(p.bank_index_key + src, key_hi | b);
-        }
-      }
-    }
-
-    // Two passes per chunk of SPs, so that the warps do not diverge between the isolated SPs
-    // (about two thirds: one pattern test each) and the neighbour scans of the others: pass 1
-    // counts the isolated SPs and queues the others (warp-aggregated), pass 2 scans the
-    // queued SPs with every lane busy.  The counts are sums, so the order does not matter.
-    const unsigned chunk = estimate_queue;
-    for (unsigned chunk_base = 0, parity = 0; chunk_base < bt.total_sp; chunk_base += chunk, parity ^= 1u) {
-      for (unsigned f = chunk_base + threadIdx.x; f < chunk_base + chunk; f += blockDim.x) {
-        bool queued = false;
-        if (f < bt.total_sp) {
-          const unsigned b = bank_of(bt, f);
-          const uint32_t word = in_smem ? held[f] : words[bt.words_off[b] + f - bt.flat[b]];
-          if (word & 0x80000000u) {
-            const unsigned mp = bank_module_pair(bt.source_id[b], p.in.bank_version);
-            if (mp < n_module_pairs) warp_aggregated_add(&est_mp[mp], mp, isolated_two_clusters(word & 0xFFu) ? 2u : 1u);
-            else set_error(p.status, err_input_capacity);
-          }
-          else {
-            queued = true;
-          }
-        }
-        const unsigned lane = threadIdx.x & 31u;
-        const unsigned mask = __ballot_sync(0xFFFFFFFFu, queued);
-        if (mask) {
-          const unsigned leader = __ffs(mask) - 1;
-          unsigned at = 0;
-          if (lane == leader) at = atomicAdd(&queue_count[parity], __popc(mask));
-          at = __shfl_sync(0xFFFFFFFFu, at, leader);
-          if (queued) queue[at + __popc(mask & ((1u << lane) - 1u))] = static_cast<uint16_t>(f - chunk_base);
-        }
-      }
-      __syncthreads();
-      const unsigned n_queued = min(queue_count[parity], chunk);
-      if (threadIdx.x == 0) queue_count[parity ^ 1u] = 0;
-      for (unsigned q = threadIdx.x; q < n_queued; q += blockDim.x) {
-        const unsigned f = chunk_base + queue[q];
-        const unsigned b = bank_of(bt, f);
-        const uint32_t* bank_words = in_smem ? held + bt.flat[b] : words + bt.words_off[b];
-        const unsigned sp_index = f - bt.flat[b];
-        const uint32_t word = bank_words[sp_index];
-        const uint32_t c = sp_candidates(word, bank_words, bt.n_sp[b]);
-        const unsigned add = ((c >> 8) & 1u) + ((c >> 24) & 1u);
-        const unsigned mp = bank_module_pair(bt.source_id[b], p.in.bank_version);
-        if (mp < n_module_pairs) warp_aggregated_add(&est_mp[mp], mp, add);
-        else set_error(p.status, err_input_capacity);
-        // places in the list for the warp's candidates: the first ones of its SPs, then the second
-        const unsigned lanes = __activemask(), lane = threadIdx.x & 31u, leader = __ffs(lanes) - 1;
-        const unsigned first = __ballot_sync(lanes, add > 0), second = __ballot_sync(lanes, add > 1);
-        unsigned at = 0;
-        if (lane == leader) at = atomicAdd(&cand_count, static_cast<unsigned>(__popc(first) + __popc(second)));
-        at = __shfl_sync(lanes, at, leader);
-        if (list != nullptr && add > 0) {
-          const uint32_t sensor =
-            v23 ? (bt.source_id[b] & 0x1FFu) : (((bt.source_id[b] & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
-          // (an SP beyond the 26 module pairs makes no cluster: a sensor that is skipped there)
-          const uint32_t code = mp < n_module_pairs ? (sp_index << 11) | (sensor << 3) : ~0u;
-          const unsigned below = (1u << lane) - 1u;
-          const unsigned one = at + __popc(first & below), two = at + __popc(first) + __popc(second & below);
-          if (one < bt.total_sp) list[one] = code | ((c & 0x100u) ? c & 0x7u : (c >> 16) & 0x7u);
-          if (add > 1 && two < bt.total_sp) list[two] = code | ((c >> 16) & 0x7u);
-          // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
-          if (mp < n_module_pairs && (sensor & 0xFFu) >= n_sensors) set_error(p.status, err_bad_sensor);
-        }
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x < n_module_pairs) {
-      p.estimated_input_size[e * n_module_pairs + threadIdx.x] = est_mp[threadIdx.x];
-    }
-    if (threadIdx.x == 0) {
-      unsigned s = 0;
-      for (unsigned mp = 0; mp < n_module_pairs; ++mp)
-        s += est_mp[mp];
-      p.event_estimate[e] = s;
-      p.number_of_candidates[e] = 2 * bt.count_total;
-      p.module_candidate_num[e] = cand_count;
-      if (p.list_scratch != nullptr) p.list_base[e] = cand_count <= bt.total_sp ? list_at : no_candidate_list;
-    }
-  }
-
-  __global__ void __launch_bounds__(decode_threads, 2048 / decode_threads) estimate_kernel(EstimateParams p)
-  {
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) mbar_init(&bar, 1);
-    __syncthreads();
-    unsigned bar_phase = 0;
-    for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { estimate_event(p, e, &bar, bar_phase); });
   }
 
   // ------------------------------------------------------------------------------------
@@ -615,16 +341,16 @@ namespace velo {
       cur = next;
       next = map & make_8con_mask(cur);
     }
+    // Sums over the pixels by bit planes of their positions (bit = 16 column + row).  Row 15
+    // counts 15 here and nothing in the reference, which drops clusters that touch it.
     PixelCluster c;
     c.pixels = cur;
-    c.n = __popcll(cur);
-    c.x = col_lower * c.n + __popcll(cur & 0x00000000FFFF0000ull) + __popcll(cur & 0x0000FFFF00000000ull) * 2 +
-          __popcll(cur & 0xFFFF000000000000ull) * 3;
-    uint32_t y = row_lower * c.n;
-#pragma unroll
-    for (unsigned r = 1; r <= 14; ++r)
-      y += __popcll(cur & (0x0001000100010001ull << r)) * r;
-    c.y = y;
+    const uint32_t lo = static_cast<uint32_t>(cur), hi = static_cast<uint32_t>(cur >> 32);
+    const unsigned n_hi = __popc(hi);
+    c.n = __popc(lo) + n_hi;
+    c.x = col_lower * c.n + __popc(lo & 0xFFFF0000u) + __popc(hi & 0xFFFF0000u) + 2 * n_hi;
+    auto plane = [&](uint32_t m) { return static_cast<unsigned>(__popc(lo & m) + __popc(hi & m)); };
+    c.y = row_lower * c.n + plane(0xAAAAAAAAu) + 2 * plane(0xCCCCCCCCu) + 4 * plane(0xF0F0F0F0u) + 8 * plane(0xFF00FF00u);
     return c;
   }
 
@@ -642,21 +368,17 @@ namespace velo {
     o.z = __ldg(ltg + 6) * local_x + __ldg(ltg + 7) * local_y + __ldg(ltg + 11);
   }
 
-  __device__ bool rest_of_clusters(
-    const Geometry* g,
-    const Constants& k,
-    uint32_t candidate,
-    const uint32_t* bank_words,
-    unsigned n_sp,
-    int version,
-    ClusterOut& o,
-    bool& bad)
+  // The cluster that a candidate grows into (MaskedVeloClustering.cu:290-459): its pixel count and
+  // the sums of their columns and rows; n = 0: none (a cluster another candidate makes, one that
+  // leaves the window, or, with bad set, no pixel at all).
+  struct ClusterSums {
+    uint32_t x, y, n;
+    bool bad;
+  };
+  __device__ __forceinline__ ClusterSums grow_cluster(
+    uint32_t sp_word, uint32_t start_loc, uint32_t sensor_number, const uint32_t* bank_words, unsigned n_sp, int version)
   {
-    const uint32_t sp_index = candidate >> 11;
-    const uint32_t sensor_number = (candidate >> 3) & 0xFFu;
-    const uint32_t start_loc = candidate & 0x7u;
-    const float* ltg = g->ltg + 12 * sensor_number;
-    const uint32_t sp_word = bank_words[sp_index];
+    ClusterSums none {0, 0, 0, false};
     const uint32_t sp_addr = (sp_word & 0x007FFF00u) >> 8;
     const int32_t sp_row = static_cast<int32_t>(sp_addr & 0x3Fu);
     const int32_t sp_col = static_cast<int32_t>(sp_addr >> 6);
@@ -696,7 +418,7 @@ namespace velo {
     const PixelCluster cl = make_cluster(map, start, static_cast<uint32_t>(col_lower + 4), static_cast<uint32_t>(row_lower));
     const uint64_t precedence = (mask_east(cl.pixels) & pa[4]) | (cl.pixels & (start ^ (0ull - start)));
     bool keep = precedence == 0 && !(cl.pixels & 0x8000800080008000ull) && !(cl.pixels & 0x0001000100010001ull);
-    if (!keep) return false;
+    if (!keep) return none;
     uint32_t x = cl.x, y = cl.y, n = cl.n;
     if (cl.pixels & 0xFFFFull) {
       const uint64_t west_map = (static_cast<uint64_t>(pa[1]) << 32) | pa[0];
@@ -709,14 +431,19 @@ namespace velo {
       keep = !(ext.pixels & 0x8000800080008000ull) && !(ext.pixels & 0xFFFFull) &&
              !(cl.pixels & 0x0001000100010001ull);
     }
-    if (!keep) return false;
+    if (!keep) return none;
     // A candidate whose bank index names another bank (the reference's lookup of the bank by
     // sensor, when a slice holds more than one bank per sensor) can leave the start pixel
     // outside the map: no pixel, and the reference divides by zero.
-    if (n == 0) {
-      bad = true;
-      return false;
-    }
+    none.bad = n == 0;
+    return n == 0 ? none : ClusterSums {x, y, n, false};
+  }
+
+  // The hit at the centroid of a candidate's cluster (MaskedVeloClustering.cu:461-496).
+  __device__ __forceinline__ void
+  candidate_cluster(const Geometry* g, const Constants& k, uint32_t sensor_number, uint32_t x, uint32_t y, uint32_t n, ClusterOut& o)
+  {
+    const float* ltg = g->ltg + 12 * sensor_number;
     // The integer centroids x / n and y / n are the truncated correctly rounded quotients: a
     // quotient below 1024 (columns < 768, rows < 256) with n < 32768 pixels is at least 1 / n
     // below the next integer, more than half an ulp, so rounding never reaches it.  The
@@ -733,7 +460,6 @@ namespace velo {
     const float local_y = (__uint2float_rn(cy) + 0.5f + fy) * 0.055f;
     local_to_global(g, ltg, local_x, local_y, o);
     o.phi = hit_phi_16(k, o.x, o.y);
-    return true;
   }
 
   // Isolated SP through the lookup tables (MaskedVeloClustering.cu:131-288); which = 0/1.
@@ -770,13 +496,211 @@ namespace velo {
     o.phi = hit_phi_16(k, o.x, o.y);
   }
 
+  constexpr unsigned estimate_queue = 1024; // SPs per chunk of the estimate (and queue entries)
+  static_assert(estimate_queue % decode_threads == 0, "every lane takes the same number of SPs per chunk");
+
+  // Items of the list an event leaves to the clustering kernel.  Isolated SP: its word's pattern,
+  // address and (version 4) sensor bit, with the bank's sensor (pair) and which of its two
+  // clusters: versions 2 and 3 which << 23 | sensor << 24, version 4 pair << 24 | which << 31.
+  // Candidate's cluster: two words, the column sum | pixel count << 24 and the row sum | sensor << 24.
+  __device__ __forceinline__ uint32_t isolated_item(uint32_t word, unsigned source_id, bool v23, unsigned which)
+  {
+    return v23 ? (word & 0x7FFFFFu) | (which << 23) | (source_id << 24) :
+                 (word & 0xFFFFFFu) | ((source_id & 0x7Fu) << 24) | (which << 31);
+  }
+
+  // ------------------------------------------------------------------------------------
+  // estimate_kernel: dev_number_of_candidates, dev_velo_bank_index (as a max-reduced
+  // key), dev_estimated_input_size and dev_module_candidate_num, and the clustering kernel's items.
+  // ------------------------------------------------------------------------------------
+  __device__ __forceinline__ void estimate_event(const EstimateParams& p, unsigned e)
+  {
+    __shared__ BankTable bt;
+    __shared__ unsigned est_mp[n_module_pairs + 6]; // zeroed by the first warp
+    __shared__ unsigned cand_count, isolated_count, grown_count;
+    __shared__ unsigned warp_sums[33];
+    __shared__ uint16_t queue[estimate_queue];
+    __shared__ uint16_t candidates[2 * estimate_queue]; // SP in the chunk, pixel << 10
+    __shared__ unsigned queue_count[2], chunk_candidates[2];
+    __shared__ unsigned list_at, no_list;
+    // the event's SPs in bank order, when they fit: the words, with the bank as its distance
+    // from the hint (127: too far) in bits 24 to 30, which SPs do not use
+    __shared__ uint32_t held[estimate_words];
+
+    const unsigned ev = e + p.in.event_start;
+    const int version = p.in.bank_version;
+    const bool v23 = version == 2 || version == 3;
+    if (threadIdx.x < 32) est_mp[threadIdx.x] = 0;
+    if (threadIdx.x == 0) cand_count = isolated_count = grown_count = no_list = 0;
+    if (threadIdx.x < 2) queue_count[threadIdx.x] = chunk_candidates[threadIdx.x] = 0;
+
+    const EventWords ew = event_words(p.in, ev);
+    const uint32_t* words = ew.w;
+    parse_banks(p.in, ev, ew, bt, warp_sums, p.status);
+    const unsigned total_sp = bt.total_sp;
+    const bool in_smem = total_sp <= estimate_words;
+    if (in_smem) {
+      for (unsigned f0 = 0; f0 < total_sp; f0 += blockDim.x) {
+        const unsigned f = f0 + threadIdx.x;
+        const unsigned b = bank_of_warp(bt, f);
+        if (f < total_sp) {
+          const uint32_t distance = min(b - bt.hint[f / 32], 127u);
+          held[f] = (words[bt.words_off[b] + f - bt.flat[b]] & 0x80FFFFFFu) | (distance << 24);
+        }
+      }
+    }
+    // Room for the event's items, two words per SP: an event that finds none, or needs more,
+    // hands over nothing.
+    const unsigned room = 2 * total_sp;
+    if (threadIdx.x == 0) {
+      list_at = no_item_list;
+      if (p.list_scratch != nullptr) {
+        const unsigned at = atomicAdd(p.list_alloc, room);
+        if (at <= p.list_capacity && room <= p.list_capacity - at) list_at = at;
+      }
+    }
+    __syncthreads();
+    uint32_t* list = list_at != no_item_list ? p.list_scratch + list_at : nullptr;
+
+    // Three passes per chunk of SPs, so that the warps do not diverge between the isolated SPs
+    // (about two thirds: one pattern test each), the neighbour scans of the others and the flood
+    // fills of the candidates: pass 1 counts and lists the isolated SPs and queues the others,
+    // pass 2 scans the queued SPs and queues their candidates, pass 3 grows the candidates'
+    // clusters.  Counts are sums and the clustering sorts, so the order does not matter.
+    auto sp_word = [&](unsigned f, unsigned& b) {
+      if (in_smem) {
+        const uint32_t w = held[f];
+        const unsigned distance = (w >> 24) & 127u;
+        b = distance < 127u ? bt.hint[f / 32] + distance : bank_of(bt, f);
+        return w;
+      }
+      b = bank_of(bt, f);
+      return words[bt.words_off[b] + f - bt.flat[b]];
+    };
+    for (unsigned chunk_base = 0, parity = 0; chunk_base < total_sp; chunk_base += estimate_queue, parity ^= 1u) {
+      for (unsigned f = chunk_base + threadIdx.x; f < min(chunk_base + estimate_queue, total_sp); f += blockDim.x) {
+        unsigned b;
+        const uint32_t word = sp_word(f, b);
+        unsigned clusters = 0;
+        if (word & 0x80000000u) {
+          const unsigned source_id = bt.source_id[b];
+          const unsigned mp = bank_module_pair(source_id, version);
+          if (mp < n_module_pairs) {
+            clusters = isolated_two_clusters(word & 0xFFu) ? 2u : 1u;
+            add_to_counter(est_mp, mp, clusters);
+            if (list != nullptr) {
+              // the sensor field of a version 2 or 3 channel id takes bit 9 of the source ID too, which
+              // an item has no room for
+              if (v23 && (source_id & 0x200u)) no_list = 1;
+              unsigned second;
+              const unsigned first = append_items(&isolated_count, clusters, second);
+              if (first < room) list[first] = isolated_item(word, source_id, v23, 0);
+              if (clusters > 1 && second < room) list[second] = isolated_item(word, source_id, v23, 1);
+            }
+          }
+          else {
+            set_error(p.status, err_input_capacity);
+          }
+        }
+        else {
+          unsigned unused;
+          queue[append_items(&queue_count[parity], 1, unused)] = static_cast<uint16_t>(f - chunk_base);
+        }
+      }
+      __syncthreads();
+      const unsigned n_queued = min(queue_count[parity], estimate_queue);
+      if (threadIdx.x == 0) queue_count[parity ^ 1u] = 0;
+      for (unsigned q = threadIdx.x; q < n_queued; q += blockDim.x) {
+        const unsigned f = chunk_base + queue[q];
+        unsigned b;
+        const uint32_t word = sp_word(f, b);
+        const unsigned at = bt.flat[b], source_id = bt.source_id[b];
+        const uint32_t* bank_words = in_smem ? held + at : words + bt.words_off[b];
+        const uint32_t c = sp_candidates(word, bank_words, bt.flat[b + 1] - at);
+        const unsigned add = ((c >> 8) & 1u) + ((c >> 24) & 1u);
+        const unsigned mp = bank_module_pair(source_id, version);
+        unsigned second;
+        const unsigned first = append_items(&chunk_candidates[parity], add, second);
+        if (add > 0)
+          candidates[first] = static_cast<uint16_t>(queue[q] | (((c & 0x100u) ? c & 0x7u : (c >> 16) & 0x7u) << 10));
+        if (add > 1) candidates[second] = static_cast<uint16_t>(queue[q] | (((c >> 16) & 0x7u) << 10));
+        if (mp < n_module_pairs) add_to_counter(est_mp, mp, add);
+        else set_error(p.status, err_input_capacity);
+      }
+      __syncthreads();
+      const unsigned n_candidates = chunk_candidates[parity];
+      if (threadIdx.x == 0) {
+        chunk_candidates[parity ^ 1u] = 0;
+        cand_count += n_candidates;
+      }
+      for (unsigned q = threadIdx.x; q < (list != nullptr ? n_candidates : 0u); q += blockDim.x) {
+        const unsigned f = chunk_base + (candidates[q] & 0x3FFu);
+        unsigned b;
+        const uint32_t word = sp_word(f, b);
+        const unsigned source_id = bt.source_id[b];
+        if (bank_module_pair(source_id, version) >= n_module_pairs) continue; // flagged above
+        // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
+        const uint32_t sensor = v23 ? (source_id & 0x1FFu) : (((source_id & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
+        const unsigned b2 = static_cast<unsigned>(p.bank_index_key[sensor] & 0xFFFFFFFFull);
+        const uint32_t* bank_words;
+        unsigned n_sp;
+        uint32_t start_word = word;
+        if (b2 == b) {
+          const unsigned at = bt.flat[b];
+          bank_words = in_smem ? held + at : words + bt.words_off[b];
+          n_sp = bt.flat[b + 1] - at;
+        }
+        else {
+          const unsigned index = f - bt.flat[b];
+          Bank bank;
+          bank.n_sp = 0;
+          if (b2 < bt.n_banks) bank = event_bank(p.in, ev, ew, b2);
+          if (index >= bank.n_sp) {
+            set_error(p.status, err_input_capacity);
+            continue;
+          }
+          bank_words = words + bank.first;
+          n_sp = bank.n_sp;
+          start_word = bank_words[index];
+        }
+        const ClusterSums c = grow_cluster(start_word, candidates[q] >> 10, sensor, bank_words, n_sp, version);
+        if (c.bad) set_error(p.status, err_bad_super_pixel);
+        if (c.n > 0) {
+          unsigned unused;
+          const unsigned at = 2 * append_items(&grown_count, 1, unused);
+          if (at + 2 <= room)
+            *reinterpret_cast<uint2*>(list + (room - 2 - at)) = make_uint2(c.x | (c.n << 24), c.y | (sensor << 24));
+        }
+      }
+      // the next chunk's first barrier comes before its candidates
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const unsigned mine = threadIdx.x < n_module_pairs ? est_mp[threadIdx.x] : 0u;
+      if (threadIdx.x < n_module_pairs) p.estimated_input_size[e * n_module_pairs + threadIdx.x] = mine;
+      const unsigned sum = __reduce_add_sync(0xFFFFFFFFu, mine);
+      if (threadIdx.x == 0) {
+        p.event_estimate[e] = sum;
+        p.number_of_candidates[e] = 2 * bt.count_total;
+        p.module_candidate_num[e] = cand_count;
+        if (p.lists != nullptr)
+          p.lists[e] = make_uint4(
+            !no_list && isolated_count + 2 * grown_count <= room ? list_at : no_item_list, room, isolated_count, grown_count);
+      }
+    }
+  }
+
+  // Issue-bound (80 % of the issue slots).  16000 events of 2540 SPs: 1.06 ms (reading and parsing
+  // 0.14, pass 1 0.24, pass 2 0.37, pass 3 0.31), where this kernel without pass 3 took 0.79 and the
+  // clustering kernel twice as long as now.
+  __global__ void __launch_bounds__(decode_threads, 2048 / decode_threads) estimate_kernel(EstimateParams p)
+  {
+    for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { estimate_event(p, e); });
+  }
+
   // ------------------------------------------------------------------------------------
   // cluster_sort_kernel
   // ------------------------------------------------------------------------------------
-  // queued candidates per chunk of 2 THREADS SPs (two candidates at most per SP)
-  template<unsigned THREADS>
-  constexpr unsigned candidate_queue = 4 * THREADS;
-
   __device__ __forceinline__ unsigned sort_bucket(int16_t phi) { return static_cast<unsigned>(phi + 32768) >> 9; }
 
   // u16 counters packed two per 32-bit word; returns the previous count of counter b.
@@ -786,24 +710,117 @@ namespace velo {
     const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(counters) + (b >> 1), 1u << shift);
     return static_cast<uint16_t>(old >> shift);
   }
-  template<unsigned THREADS>
-  __device__ __forceinline__ void
-  cluster_sort_event(const ClusterSortParams& p, unsigned e, uint64_t* bar, unsigned& bar_phase)
-  {
-    constexpr unsigned queue_size = candidate_queue<THREADS>;
-    extern __shared__ __align__(128) unsigned char dsmem[];
-    __shared__ BankTable bt;
-    __shared__ unsigned region[n_module_pairs + 1]; // estimated start of each module pair, event-relative
-    __shared__ unsigned mp_count[n_module_pairs];
-    __shared__ unsigned staged_first[n_module_pairs + 1]; // staged clusters before each module pair
-    __shared__ unsigned warp_sums[33];
-    __shared__ unsigned sorted_total;
-    __shared__ uint32_t queue[queue_size];
-    __shared__ unsigned queue_count[2];
 
+  // The clusters of an event as they are made (22 bytes each), in shared memory or in the event's
+  // slice of the global staging buffer.
+  struct StagedClusters {
+    uint4* hit;        // x, y, z, id
+    uint32_t* key;     // phi, module pair << 16
+    uint16_t* members; // cluster indices in bucket order
+    __device__ __forceinline__ StagedClusters(char* base, unsigned capacity)
+    {
+      hit = reinterpret_cast<uint4*>(base);
+      key = reinterpret_cast<uint32_t*>(hit + capacity);
+      members = reinterpret_cast<uint16_t*>(key + capacity);
+    }
+  };
+
+  struct ClusterSortShared {
+    unsigned region[n_module_pairs + 1]; // estimated start of each module pair, event-relative
+    unsigned n_staged;
+    unsigned warp_sums[33];
+  };
+
+  // Makes clusters and appends them to the event's staging.
+  struct ClusterMaker {
+    const ClusterSortParams& p;
+    const StagedClusters& st;
+    ClusterSortShared& s;
+    uint16_t* counters;
+    unsigned est_total;
+
+    __device__ __forceinline__ void stage(const ClusterOut& o, unsigned mp) const
+    {
+      unsigned unused;
+      const unsigned k = append_items(&s.n_staged, 1, unused);
+      if (k < est_total) {
+        st.hit[k] = make_uint4(__float_as_uint(o.x), __float_as_uint(o.y), __float_as_uint(o.z), o.id);
+        st.key[k] = static_cast<uint16_t>(o.phi) | (mp << 16);
+        count_in_bucket(counters, mp * sort_buckets + sort_bucket(o.phi));
+      }
+      else {
+        set_error(p.status, err_cluster_capacity);
+      }
+    }
+    __device__ __forceinline__ void isolated(uint32_t word, unsigned source_id, unsigned which) const
+    {
+      ClusterOut o;
+      isolated_cluster(p.geo, p.k, word, source_id, p.in.bank_version, which, o);
+      stage(o, bank_module_pair(source_id, p.in.bank_version));
+    }
+    __device__ __forceinline__ void grown(uint32_t x, uint32_t y, uint32_t n, uint32_t sensor) const
+    {
+      ClusterOut o;
+      candidate_cluster(p.geo, p.k, sensor, x, y, n, o);
+      stage(o, sensor / 8);
+    }
+  };
+
+  // The clusters of an event without an item list (its list found no room, two clusters from
+  // too many of its SPs, or source IDs an item cannot hold): a thread per bank.
+  __device__ __noinline__ void
+  cluster_banks(const ClusterSortParams& p, char* stage_base, ClusterSortShared& s, uint16_t* counters, unsigned est_total, unsigned e)
+  {
+    const StagedClusters st {stage_base, est_total};
+    const ClusterMaker m {p, st, s, counters, est_total};
     const unsigned ev = e + p.in.event_start;
-    const unsigned n = p.in.n_events;
+    const EventWords ew = event_words(p.in, ev);
     const int version = p.in.bank_version;
+    const bool v23 = version == 2 || version == 3;
+    for (unsigned b = threadIdx.x; b < ew.n_banks; b += blockDim.x) {
+      const Bank bank = event_bank(p.in, ev, ew, b);
+      // a source id beyond the 26 module pairs: malformed input, flagged by estimate_kernel
+      if (!bank.velo || bank_module_pair(bank.source_id, version) >= n_module_pairs) continue;
+      const uint32_t* w = ew.w + bank.first;
+      for (unsigned i = 0; i < bank.n_sp; ++i) {
+        const uint32_t word = w[i];
+        if (word & 0x80000000u) {
+          const unsigned clusters = isolated_two_clusters(word & 0xFFu) ? 2u : 1u;
+          for (unsigned which = 0; which < clusters; ++which)
+            m.isolated(word, bank.source_id, which);
+          continue;
+        }
+        const uint32_t c = sp_candidates(word, w, bank.n_sp);
+        const uint32_t sensor =
+          v23 ? (bank.source_id & 0x1FFu) : (((bank.source_id & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
+        // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
+        const unsigned b2 = static_cast<unsigned>(p.bank_index_key[sensor] & 0xFFFFFFFFull);
+        Bank at;
+        at.n_sp = 0;
+        if (b2 < ew.n_banks) at = event_bank(p.in, ev, ew, b2);
+        for (unsigned which = 0; which < 2; ++which) {
+          const uint32_t code = which ? (c >> 16) : c;
+          if (!(code & 0x100u)) continue;
+          if (i >= at.n_sp) {
+            set_error(p.status, err_input_capacity);
+            continue;
+          }
+          const uint32_t* w2 = ew.w + at.first;
+          const ClusterSums sums = grow_cluster(w2[i], code & 0x7u, sensor, w2, at.n_sp, version);
+          if (sums.bad) set_error(p.status, err_bad_super_pixel);
+          if (sums.n > 0) m.grown(sums.x, sums.y, sums.n, sensor);
+        }
+      }
+    }
+  }
+
+  template<unsigned THREADS>
+  __device__ __forceinline__ void cluster_sort_event(const ClusterSortParams& p, unsigned e)
+  {
+    extern __shared__ __align__(128) unsigned char dsmem[];
+    __shared__ ClusterSortShared s;
+
+    const unsigned n = p.in.n_events;
     const unsigned base = p.event_base[e];
     const unsigned T = p.event_base[n];
     if (T > p.cluster_capacity) {
@@ -811,261 +828,173 @@ namespace velo {
       if (threadIdx.x == 0) set_error(p.status, err_input_capacity);
       return;
     }
-
-    if (threadIdx.x == 0) {
-      unsigned s = 0;
-      for (unsigned mp = 0; mp < n_module_pairs; ++mp) {
-        region[mp] = s;
-        s += p.estimated_input_size[e * n_module_pairs + mp];
+    if (threadIdx.x < 32) {
+      const unsigned mp = threadIdx.x;
+      const unsigned mine = mp < n_module_pairs ? p.estimated_input_size[e * n_module_pairs + mp] : 0u;
+      unsigned incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (mp >= static_cast<unsigned>(o)) incl += t;
       }
-      region[n_module_pairs] = s;
+      if (mp <= n_module_pairs) s.region[mp] = incl - mine;
+      if (mp < n_module_pairs) p.offsets_estimated_input_size[e * n_module_pairs + mp] = base + incl - mine;
+      if (mp == 0) s.n_staged = 0;
+      if (e == n - 1 && mp == 0) p.offsets_estimated_input_size[n * n_module_pairs] = T;
     }
-    if (threadIdx.x < n_module_pairs) mp_count[threadIdx.x] = 0;
-    if (threadIdx.x < 2) queue_count[threadIdx.x] = 0;
-    __syncthreads();
-    if (threadIdx.x < n_module_pairs) {
-      p.offsets_estimated_input_size[e * n_module_pairs + threadIdx.x] = base + region[threadIdx.x];
-    }
-    if (e == n - 1 && threadIdx.x == 0) p.offsets_estimated_input_size[n * n_module_pairs] = T;
-
-    const unsigned est_total = region[n_module_pairs];
-    // Staging of the unsorted clusters (18 bytes each) plus two u16 per cluster for the
-    // sort: shared memory when they fit, else the event's slice of the global staging
-    // buffer (24 bytes per estimated cluster).  Bucket counters and the blob follow.
-    const bool staged_in_smem = est_total <= p.smem_cluster_capacity;
-    const unsigned cap = staged_in_smem ? p.smem_cluster_capacity : est_total;
-    char* stage_base = staged_in_smem ? reinterpret_cast<char*>(dsmem) : p.staging + size_t(24) * base;
-    ClusterView st {stage_base, est_total};
-    uint16_t* slot_in_bucket = reinterpret_cast<uint16_t*>(stage_base + size_t(element_size) * cap);
-    uint16_t* members = slot_in_bucket + cap;
-    uint16_t* bucket_start = reinterpret_cast<uint16_t*>(dsmem + cluster_sort_counter_offset(p.smem_cluster_capacity));
-    unsigned char* blob = dsmem + cluster_sort_blob_offset(p.smem_cluster_capacity);
+    uint16_t* bucket = reinterpret_cast<uint16_t*>(dsmem + cluster_sort_counter_offset(p.smem_cluster_capacity));
     for (unsigned i = threadIdx.x; i < sort_counters / 2; i += blockDim.x)
-      reinterpret_cast<uint32_t*>(bucket_start)[i] = 0;
+      reinterpret_cast<uint32_t*>(bucket)[i] = 0;
+    __syncthreads();
 
-    unsigned n_words, staged;
-    const uint32_t* words = stage_event(p.in, ev, blob, p.smem_blob_bytes, bar, bar_phase, p.status, n_words, staged);
-    parse_banks(p.in, ev, words, n_words, bt, warp_sums, p.status);
-    index_banks(bt);
-    // the candidates the estimate kernel found, unless it left none
-    const unsigned list_at = p.list_base != nullptr ? p.list_base[e] : no_candidate_list;
-    const uint32_t* list = list_at != no_candidate_list ? p.list_scratch + list_at : nullptr;
+    // Staging: shared memory when the event fits (always the smallest), else its slice of the
+    // global staging buffer (24 bytes per estimated cluster), from a 16-byte boundary on.
+    const unsigned est_total = s.region[n_module_pairs];
+    const bool staged_in_smem = est_total <= p.smem_cluster_capacity;
+    char* stage_base = staged_in_smem ? reinterpret_cast<char*>(dsmem) : p.staging + ((size_t(24) * base + 15) & ~size_t(15));
+    const StagedClusters st {stage_base, est_total};
 
-    const Geometry* g = p.geo;
-    auto stage_cluster = [&](const ClusterOut& o, unsigned mp) {
-      const unsigned slot = warp_aggregated_inc(&mp_count[mp], mp);
-      if (region[mp] + slot < region[mp + 1]) {
-        const unsigned i = region[mp] + slot;
-        st.id(i) = o.id;
-        st.x(i) = o.x;
-        st.y(i) = o.y;
-        st.z(i) = o.z;
-        st.phi(i) = o.phi;
-        slot_in_bucket[i] = count_in_bucket(bucket_start, mp * sort_buckets + sort_bucket(o.phi));
+    const uint4 items = p.lists != nullptr ? p.lists[e] : make_uint4(no_item_list, 0, 0, 0);
+    if (items.x != no_item_list) {
+      // the isolated SPs from the front, the candidates' clusters from the end
+      const ClusterMaker make {p, st, s, bucket, est_total};
+      const uint32_t* list = p.list_scratch + items.x;
+      const bool v23 = p.in.bank_version == 2 || p.in.bank_version == 3;
+      for (unsigned q = threadIdx.x; q < items.z; q += blockDim.x) {
+        const uint32_t item = __ldcs(list + q);
+        if (v23) make.isolated(item & 0x7FFFFFu, item >> 24, (item >> 23) & 1u);
+        else make.isolated(item & 0xFFFFFFu, (item >> 24) & 0x7Fu, item >> 31);
       }
-      else {
-        set_error(p.status, err_cluster_capacity);
+      const uint2* grown = reinterpret_cast<const uint2*>(list + items.y) - 1;
+      for (unsigned q = threadIdx.x; q < items.w; q += blockDim.x) {
+        const uint2 g = __ldcs(grown - q);
+        make.grown(g.x & 0xFFFFFFu, g.y & 0xFFFFFFu, g.x >> 24, g.y >> 24);
       }
-    };
-
-    // The cluster of a candidate, by the reference in the bank that its table names for the
-    // sensor.
-    auto cluster_candidate = [&](uint32_t candidate) {
-      const uint32_t cand_sensor = (candidate >> 3) & 0xFFu;
-      if (cand_sensor >= n_sensors) return; // flagged where the candidate was found
-      const unsigned b2 = static_cast<unsigned>(p.bank_index_key[cand_sensor] & 0xFFFFFFFFull);
-      if (b2 >= bt.n_banks || (candidate >> 11) >= bt.n_sp[b2]) {
-        set_error(p.status, err_input_capacity);
-        return;
-      }
-      ClusterOut o;
-      bool bad = false;
-      if (rest_of_clusters(g, p.k, candidate, words + bt.words_off[b2], bt.n_sp[b2], version, o, bad))
-        stage_cluster(o, cand_sensor / 8);
-      else if (bad)
-        set_error(p.status, err_bad_super_pixel);
-    };
-
-    // Isolated SPs (about two thirds, one table lookup each) and candidates (flood fills) in
-    // passes of their own, so that the warps do not diverge between them: the isolated ones
-    // over the event's SPs, the candidates over the estimate kernel's list.  Without a list
-    // the other SPs are searched again, in chunks of queue_size / 2 SPs: their candidates
-    // (EstimateInputSize.cu:72-204 order of codes) are queued, and clustered after each chunk
-    // (the queue cannot overflow; every lane takes the same number of SPs per chunk).
-    const unsigned chunk = list ? bt.total_sp : queue_size / 2;
-    for (unsigned chunk_base = 0, parity = 0; chunk_base < bt.total_sp; chunk_base += chunk, parity ^= 1u) {
-      for (unsigned f0 = chunk_base; f0 < min(chunk_base + chunk, bt.total_sp); f0 += blockDim.x) {
-        const unsigned f = f0 + threadIdx.x;
-        uint32_t cand[2] = {0, 0};
-        bool valid[2] = {false, false};
-        if (f < bt.total_sp) {
-          const unsigned b = bank_of(bt, f);
-          const unsigned mp = bank_module_pair(bt.source_id[b], version);
-          const uint32_t* bank_words = words + bt.words_off[b];
-          const unsigned sp_index = f - bt.flat[b];
-          const uint32_t word = bank_words[sp_index];
-          if (mp >= n_module_pairs) {
-            // a source id beyond the 26 module pairs: malformed input, flagged by estimate_kernel
-          }
-          else if (word & 0x80000000u) {
-            const unsigned n_clusters = (__ldg(g->sp_patterns + (word & 0xFFu)) & 8u) ? 2u : 1u;
-            for (unsigned which = 0; which < n_clusters; ++which) {
-              ClusterOut o;
-              isolated_cluster(g, p.k, word, bt.source_id[b], version, which, o);
-              stage_cluster(o, mp);
-            }
-          }
-          else if (!list) {
-            const uint32_t c = sp_candidates(word, bank_words, bt.n_sp[b]);
-            const bool v23 = version == 2 || version == 3;
-            const uint32_t sensor_number =
-              v23 ? (bt.source_id[b] & 0x1FFu) : (((bt.source_id[b] & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
-            for (unsigned which = 0; which < 2; ++which) {
-              const uint32_t code = which ? (c >> 16) : c;
-              if (!(code & 0x100u)) continue;
-              cand[which] = (sp_index << 11) | (sensor_number << 3) | (code & 0x7u);
-              // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
-              if (((cand[which] >> 3) & 0xFFu) >= n_sensors) set_error(p.status, err_bad_sensor);
-              else valid[which] = true;
-            }
-          }
-        }
-        if (list) continue;
-        // warp-aggregated append to the queue (every lane of the warp gets here)
-        const unsigned lane = threadIdx.x & 31u;
-        for (unsigned which = 0; which < 2; ++which) {
-          const unsigned mask = __ballot_sync(0xFFFFFFFFu, valid[which]);
-          if (mask == 0) continue;
-          const unsigned leader = __ffs(mask) - 1;
-          unsigned at = 0;
-          if (lane == leader) at = atomicAdd(&queue_count[parity], __popc(mask));
-          at = __shfl_sync(0xFFFFFFFFu, at, leader);
-          if (valid[which]) queue[at + __popc(mask & ((1u << lane) - 1u))] = cand[which];
-        }
-      }
-      if (!list) __syncthreads();
-      const unsigned queued = list ? p.module_candidate_num[e] : min(queue_count[parity], queue_size);
-      if (!list && threadIdx.x == 0) queue_count[parity ^ 1u] = 0;
-      for (unsigned q = threadIdx.x; q < queued; q += blockDim.x)
-        cluster_candidate(list ? __ldcs(list + q) : queue[q]);
-      __syncthreads();
     }
+    else {
+      cluster_banks(p, stage_base, s, bucket, est_total, e);
+    }
+    __syncthreads();
 
     // Sort by (phi, id) inside each module pair (SortByPhi.cu:104-122).  The reference
     // ranks every pair of clusters; here clusters were counted into 128 phi buckets per
     // module pair while staged, so a scan of the counters places every bucket and a
     // cluster's rank is its bucket's start plus the number of smaller (phi, id) keys in the
     // same bucket - the same position as the reference's full count.
+    const unsigned n_staged = min(s.n_staged, est_total);
     {
-      // each thread owns `per` consecutive counters: it sums them, and after the scan turns
-      // them into starts in place (no other thread reads them in between)
-      constexpr unsigned per = (sort_counters + THREADS - 1) / THREADS;
+      // each thread owns `per` consecutive words of two counters: it sums them, and after the
+      // scan turns them into starts in place (no other thread reads them in between)
+      constexpr unsigned words = sort_counters / 2, per = (words + THREADS - 1) / THREADS;
+      uint32_t* w = reinterpret_cast<uint32_t*>(bucket) + threadIdx.x * per;
       unsigned sum = 0;
+#pragma unroll
       for (unsigned q = 0; q < per; ++q) {
-        const unsigned b = threadIdx.x * per + q;
-        if (b < sort_counters) sum += bucket_start[b];
+        const uint32_t c = threadIdx.x * per + q < words ? w[q] : 0u;
+        sum += (c & 0xFFFFu) + (c >> 16);
       }
       unsigned total;
-      unsigned excl = block_exclusive_scan(sum, warp_sums, &total);
-      if (threadIdx.x == 0) {
-        sorted_total = total;
-        unsigned staged = 0;
-        for (unsigned mp = 0; mp < n_module_pairs; ++mp) {
-          staged_first[mp] = staged;
-          staged += min(mp_count[mp], region[mp + 1] - region[mp]);
-        }
-        staged_first[n_module_pairs] = staged;
-      }
+      unsigned start = block_exclusive_scan(sum, s.warp_sums, &total);
+#pragma unroll
       for (unsigned q = 0; q < per; ++q) {
-        const unsigned b = threadIdx.x * per + q;
-        if (b < sort_counters) {
-          const unsigned count = bucket_start[b];
-          bucket_start[b] = static_cast<uint16_t>(excl);
-          excl += count;
+        if (threadIdx.x * per + q < words) {
+          const uint32_t c = w[q];
+          w[q] = (start & 0xFFFFu) | ((start + (c & 0xFFFFu)) << 16);
+          start += (c & 0xFFFFu) + (c >> 16);
         }
       }
     }
     __syncthreads();
-    // the k-th staged cluster of the event: its module pair (the last one whose first staged
-    // cluster is at most k, empty ones skipped) and its staging index
-    const unsigned n_staged = staged_first[n_module_pairs];
-    auto module_pair_of = [&](unsigned k) {
-      unsigned lo = 0, hi = n_module_pairs;
-      while (hi - lo > 1) {
-        const unsigned mid = (lo + hi) / 2;
-        if (staged_first[mid] <= k) lo = mid;
-        else hi = mid;
-      }
-      return lo;
+    auto bucket_of_key = [&](uint32_t key) {
+      return (key >> 16) * sort_buckets + sort_bucket(static_cast<int16_t>(key & 0xFFFFu));
     };
-    for (unsigned k = threadIdx.x; k < n_staged; k += blockDim.x) {
-      const unsigned mp = module_pair_of(k);
-      const unsigned i = region[mp] + (k - staged_first[mp]);
-      const unsigned b = mp * sort_buckets + sort_bucket(st.phi(i));
-      const unsigned q = bucket_start[b] + slot_in_bucket[i];
-      if (q < cap) members[q] = static_cast<uint16_t>(i);
-    }
+    // each cluster into its bucket; this moves a bucket's start to its end
+    for (unsigned k = threadIdx.x; k < n_staged; k += blockDim.x)
+      st.members[count_in_bucket(bucket, bucket_of_key(st.key[k]))] = static_cast<uint16_t>(k);
     __syncthreads();
+    // In bucket order, which is output order up to the order inside a bucket: the threads of a
+    // warp write neighbouring places of the container.
+    auto bucket_begin = [&](unsigned b) { return b ? unsigned(bucket[b - 1]) : 0u; };
     ClusterView out {p.sorted_container, T};
-    for (unsigned k = threadIdx.x; k < n_staged; k += blockDim.x) {
-      const unsigned mp = module_pair_of(k);
-      const unsigned i = region[mp] + (k - staged_first[mp]);
-      const unsigned count = staged_first[mp + 1] - staged_first[mp];
-      const int16_t phi = st.phi(i);
-      const uint32_t id = st.id(i);
-      const unsigned b = mp * sort_buckets + sort_bucket(phi);
-      const unsigned b_end = min(b + 1 < sort_counters ? unsigned(bucket_start[b + 1]) : sorted_total, cap);
-      unsigned position = bucket_start[b] - bucket_start[mp * sort_buckets];
-      for (unsigned q = bucket_start[b]; q < b_end; ++q) {
-        const unsigned j = members[q];
-        if (j == i || j >= est_total) continue;
-        const int16_t other = st.phi(j);
-        position += phi > other || (phi == other && id > st.id(j));
+    for (unsigned q = threadIdx.x; q < n_staged; q += blockDim.x) {
+      const unsigned k = st.members[q];
+      const uint32_t key = st.key[k];
+      const uint4 hit = st.hit[k];
+      const unsigned mp = key >> 16, b = bucket_of_key(key);
+      const int16_t phi = static_cast<int16_t>(key & 0xFFFFu);
+      const unsigned begin = bucket_begin(b), end = bucket[b];
+      unsigned position = begin - bucket_begin(mp * sort_buckets);
+      for (unsigned r = begin; r < end; ++r) {
+        const unsigned j = st.members[r];
+        const int16_t other = static_cast<int16_t>(st.key[j] & 0xFFFFu);
+        position += phi > other || (phi == other && hit.w > st.hit[j].w);
       }
-      if (position >= count) {
+      if (position >= s.region[mp + 1] - s.region[mp]) {
         set_error(p.status, err_cluster_capacity);
         continue;
       }
       // written once here, read by the next kernel: streaming stores (evict first), which
       // leave L2 to the staging of the events in flight
-      const unsigned dst = base + region[mp] + position;
-      __stcs(&out.id(dst), id);
+      const unsigned dst = base + s.region[mp] + position;
+      __stcs(&out.id(dst), hit.w);
       __stcs(&out.phi(dst), phi);
-      __stcs(&out.x(dst), st.x(i));
-      __stcs(&out.y(dst), st.y(i));
-      __stcs(&out.z(dst), st.z(i));
+      __stcs(&out.x(dst), __uint_as_float(hit.x));
+      __stcs(&out.y(dst), __uint_as_float(hit.y));
+      __stcs(&out.z(dst), __uint_as_float(hit.z));
     }
     if (threadIdx.x < n_module_pairs) {
       const unsigned mp = threadIdx.x;
-      p.module_cluster_num[e * n_module_pairs + mp] = staged_first[mp + 1] - staged_first[mp];
+      const unsigned made = bucket[(mp + 1) * sort_buckets - 1] - bucket_begin(mp * sort_buckets);
+      p.module_cluster_num[e * n_module_pairs + mp] = min(made, s.region[mp + 1] - s.region[mp]);
     }
-    // the event's slices of the global staging and of the candidate list are dead
+    // the event's slices of the global staging and of the item list are dead
     __syncthreads();
-    if (!staged_in_smem) discard_l2(stage_base, size_t(24) * est_total);
-    if (list) discard_l2(list, size_t(4) * bt.total_sp);
+    if (!staged_in_smem) discard_l2(stage_base, size_t(22) * est_total);
+    if (items.x != no_item_list) discard_l2(p.list_scratch + items.x, size_t(4) * items.y);
   }
 
-  // Capped for 2048 threads per SM (32 registers, no spills: eight 256-thread CTAs, or
-  // twelve 128-thread ones where shared memory ends them): with the clusters staged through L2
-  // (cluster_stage_capacity 0) and no event staging (cluster_blob_bytes 0) shared memory allows
-  // that many; measured 2.59 -> 2.21 -> 2.13 ms per launch from six CTAs with staging.
+  // Issue- and latency-bound.  16000 events of 2540 SPs: 0.65 ms, of which making the clusters 0.2
+  // and the sort 0.38; with the flood fills and the search for each SP's bank in this kernel, and
+  // the clusters written out in the order they were staged, 1.31 ms.  Written out from a staging
+  // without any order (a scattered store per value) the sort alone took 0.91 ms.
+  // Capped for 2048 threads per SM (32 registers; 40 or 48 registers: 0.69, 0.71 ms).
   template<unsigned THREADS>
-  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) cluster_sort_kernel(ClusterSortParams p)
+  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) cluster_sort_kernel(const __grid_constant__ ClusterSortParams p)
   {
     static_assert(THREADS == 128 || THREADS == 256, "block size");
-    __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) mbar_init(&bar, 1);
-    __syncthreads();
-    unsigned bar_phase = 0;
-    for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { cluster_sort_event<THREADS>(p, e, &bar, bar_phase); });
+    for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { cluster_sort_event<THREADS>(p, e); });
   }
-  template __global__ void cluster_sort_kernel<128>(ClusterSortParams p);
-  template __global__ void cluster_sort_kernel<256>(ClusterSortParams p);
+  template __global__ void cluster_sort_kernel<128>(const __grid_constant__ ClusterSortParams p);
+  template __global__ void cluster_sort_kernel<256>(const __grid_constant__ ClusterSortParams p);
 
-  // Events of the slice by raw size, largest first: a counting sort over 1024 size classes
-  // of 64 bytes (order within a class is arbitrary).  One CTA of scan_threads threads.
-  __global__ void __launch_bounds__(scan_threads) event_order_kernel(RawInput in, unsigned* order)
+  // Before the estimate kernel.  Block 0: the events of the slice by raw size, largest first (a
+  // counting sort over 1024 size classes of 64 bytes; order within a class is arbitrary), when
+  // order is given.  Block 1 + d: dev_velo_bank_index, as a max-reduced key, from event
+  // d * stride: block 0 of the reference's velo_calculate_number_of_candidates (grid of
+  // ceil(N / 256) blocks, one thread per event) handles events 0, stride, 2 stride, ... and the
+  // last of them to write an entry wins.
+  __global__ void __launch_bounds__(scan_threads)
+  event_order_kernel(RawInput in, unsigned* order, unsigned stride, unsigned long long* bank_index_key)
   {
+    if (blockIdx.x > 0) {
+      const unsigned e = (blockIdx.x - 1) * stride;
+      if (e >= in.n_events) return;
+      const unsigned ev = e + in.event_start;
+      const EventWords ew = event_words(in, ev);
+      const unsigned long long key_hi = static_cast<unsigned long long>(e) << 32;
+      for (unsigned b = threadIdx.x; b < ew.n_banks; b += blockDim.x) {
+        const unsigned src = event_bank(in, ev, ew, b).source_id & 0x1FFu;
+        if (in.bank_version > 3) {
+          if ((src << 1) < n_sensors) atomicMax(bank_index_key + (src << 1), key_hi | b);
+          if (((src << 1) | 1u) < n_sensors) atomicMax(bank_index_key + ((src << 1) | 1u), key_hi | b);
+        }
+        else if (src < n_sensors) {
+          atomicMax(bank_index_key + src, key_hi | b);
+        }
+      }
+      return;
+    }
+    if (order == nullptr) return;
     constexpr unsigned classes = 1024;
     __shared__ unsigned count[classes];
     __shared__ unsigned warp_sums[33];

@@ -50,21 +50,19 @@ namespace velo {
     unsigned* number_of_candidates;       // [N]    dev_number_of_candidates
     unsigned* module_candidate_num;       // [N]    dev_module_candidate_num
     unsigned* event_estimate;             // [N]    sum of the event's 26 estimates
-    unsigned long long* bank_index_key;   // [208]  (event << 32 | bank), max-reduced
-    unsigned designated_stride;           // events e with e % stride == 0 set the bank index
+    const unsigned long long* bank_index_key; // [208] (event << 32 | bank), max-reduced
     unsigned* status;
-    unsigned smem_blob_bytes;
-    // the candidates this kernel finds, for the clustering kernel (null: none are handed over):
-    // each event takes total_sp words of list_scratch from the counter list_alloc (zeroed before
-    // the launch) and records where in list_base[e] (no_candidate_list: no room, or too many)
+    // the clusters to make, an item each, for the clustering kernel (null: none are handed over):
+    // each event takes two words per SP of list_scratch from the counter list_alloc (zeroed before
+    // the launch) and records them in lists[e]
     uint32_t* list_scratch;
     unsigned list_capacity;
     unsigned* list_alloc;
-    unsigned* list_base;
+    uint4* lists; // [N] first word (no_item_list: no room, or too many), words, isolated items, grown clusters
     WorkQueue queue;
   };
 
-  constexpr unsigned no_candidate_list = 0xFFFFFFFFu;
+  constexpr unsigned no_item_list = 0xFFFFFFFFu;
 
   // ---- masked clustering + phi + sort by phi, one event per CTA ----
   struct ClusterSortParams {
@@ -78,11 +76,9 @@ namespace velo {
     unsigned* module_cluster_num;               // [26 N]     dev_module_cluster_num
     char* sorted_container;                     // [18 T]     dev_sorted_velo_cluster_container
     char* staging;                              // [24 T]     fallback staging for large events
-    const uint32_t* list_scratch;               // the estimate kernel's candidates: module_candidate_num[e]
-    const unsigned* list_base;                  // [N]  words from list_base[e] on (null: found again here)
-    const unsigned* module_candidate_num;       // [N]
+    const uint32_t* list_scratch;               // the estimate kernel's items
+    const uint4* lists;                         // [N] where an event's items lie (null: no lists)
     unsigned* status;
-    unsigned smem_blob_bytes;
     unsigned smem_cluster_capacity;             // clusters staged in shared memory per event
     unsigned cluster_capacity;                  // allocated T of the containers
     WorkQueue queue;
@@ -157,21 +153,23 @@ namespace velo {
   };
 
   // Dynamic shared memory of cluster_sort_kernel for a staging capacity of `cap` clusters:
-  // [cap x 18 B clusters][cap x u16 slot in bucket][cap x u16 members][u16 bucket counters][blob]
+  // [cap x 22 B clusters][u16 bucket counters]
   constexpr unsigned sort_buckets = 128;
   constexpr unsigned sort_counters = n_module_pairs * sort_buckets;
   __host__ __device__ constexpr unsigned cluster_sort_counter_offset(unsigned cap)
   {
     return ((cap * (element_size + 4)) + 15u) & ~15u;
   }
-  __host__ __device__ constexpr unsigned cluster_sort_blob_offset(unsigned cap)
+  // least capacity: the global staging has no room for the alignment of fewer than 4 clusters
+  constexpr unsigned min_cluster_stage = 64;
+  __host__ __device__ constexpr unsigned cluster_sort_smem(unsigned cap)
   {
     return cluster_sort_counter_offset(cap) + ((sort_counters * 2 + 15u) & ~15u);
   }
 
   __global__ void estimate_kernel(EstimateParams p);
   template<unsigned THREADS> // 128 or 256
-  __global__ void cluster_sort_kernel(ClusterSortParams p);
+  __global__ void cluster_sort_kernel(const __grid_constant__ ClusterSortParams p);
   template<unsigned THREADS, unsigned LPH, unsigned RING>
   __global__ void search_by_triplet_kernel(SearchParams p);
   // flat seeding behind the learned seed gate (and seed-candidate outcome recording);
@@ -241,8 +239,13 @@ namespace velo {
   };
   __global__ void export_half_kernel(HalfExportParams p);
 
-  // order[0..n) = the slice's events by raw size, largest first (one CTA)
-  __global__ void event_order_kernel(RawInput in, unsigned* order);
+  // order[0..n) = the slice's events by raw size, largest first, and the bank index
+  __global__ void event_order_kernel(RawInput in, unsigned* order, unsigned stride, unsigned long long* bank_index_key);
+  inline unsigned bank_index_stride(unsigned n) { return (n + 255) / 256; }
+  inline unsigned event_order_grid(unsigned n, bool bank_index)
+  {
+    return 1 + (bank_index ? (n + bank_index_stride(n) - 1) / bank_index_stride(n) : 0u);
+  }
   __global__ void exclusive_scan_kernel(ScanParams p);
 
   // Phi buckets of a module pair's sorted hits, shared by the search and the seed gate:

@@ -44,18 +44,19 @@ namespace {
   constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
   constexpr size_t off_bank_index = 0;
   constexpr size_t off_status = align256(off_bank_index + velo::n_sensors * sizeof(unsigned long long));
-  constexpr size_t off_estimated = align256(off_status + sizeof(unsigned));
+  constexpr size_t off_list_alloc = off_status + sizeof(unsigned); // zeroed with the status word
+  constexpr size_t off_estimated = align256(off_list_alloc + sizeof(unsigned));
   constexpr size_t off_n_candidates = align256(off_estimated + size_t(velo::n_module_pairs) * max_events * 4);
   constexpr size_t off_candidate_num = align256(off_n_candidates + size_t(max_events) * 4);
   constexpr size_t off_event_estimate = align256(off_candidate_num + size_t(max_events) * 4);
   constexpr size_t off_event_base = align256(off_event_estimate + size_t(max_events) * 4);
   constexpr size_t off_candidates_offsets = align256(off_event_base + size_t(max_events + 1) * 4);
   constexpr size_t off_staging = align256(off_candidates_offsets + size_t(max_events + 1) * 4);
-  constexpr size_t scratch_bytes = align256(off_staging + size_t(24) * max_clusters);
+  constexpr size_t off_list = align256(off_staging + size_t(24) * max_clusters);
+  constexpr size_t off_lists = align256(off_list + size_t(4) * max_clusters);
+  constexpr size_t scratch_bytes = align256(off_lists + size_t(max_events) * sizeof(uint4));
   static_assert(scratch_bytes <= 8u * 1024 * 1024, "scratch array above its stated 8 MiB");
 
-  constexpr unsigned estimate_blob_bytes = 32 * 1024;
-  constexpr unsigned cluster_blob_bytes = 16 * 1024;
   constexpr unsigned cluster_stage_capacity = 3072;
 
   std::mutex setup_mutex;
@@ -87,10 +88,8 @@ namespace {
       void* ptr = nullptr;
       const cudaError_t e = cudaGetSymbolAddress(&ptr, velo_noalloc_scratch);
       if (e != cudaSuccess) return fail(VELO_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-      const int cluster_smem = int(velo::cluster_sort_blob_offset(cluster_stage_capacity) + cluster_blob_bytes);
-      if (velo::raise_dynamic_smem_limit(reinterpret_cast<const void*>(velo::estimate_kernel), int(estimate_blob_bytes)) !=
-            cudaSuccess ||
-          velo::raise_dynamic_smem_limit(reinterpret_cast<const void*>(velo::cluster_sort_kernel<velo::decode_threads>), cluster_smem) !=
+      const int cluster_smem = int(velo::cluster_sort_smem(cluster_stage_capacity));
+      if (velo::raise_dynamic_smem_limit(reinterpret_cast<const void*>(velo::cluster_sort_kernel<velo::decode_threads>), cluster_smem) !=
             cudaSuccess)
         return fail(VELO_ERR_CUDA, "cannot set the kernels' shared-memory limits");
       scratch_address[device] = static_cast<unsigned char*>(ptr);
@@ -170,9 +169,9 @@ VeloStatus velo_decode_noalloc(
   auto* candidates_offsets = reinterpret_cast<unsigned*>(scratch + off_candidates_offsets);
   char* staging = reinterpret_cast<char*>(scratch + off_staging);
 
-  // what must start at zero: the max-reduced bank index and the status word
+  // what must start at zero: the max-reduced bank index, the status word and the list counter
   if (cudaMemsetAsync(bank_index, 0, n_sensors * sizeof(unsigned long long), stream) != cudaSuccess ||
-      cudaMemsetAsync(status, 0, sizeof(unsigned), stream) != cudaSuccess)
+      cudaMemsetAsync(status, 0, 2 * sizeof(unsigned), stream) != cudaSuccess)
     return fail(VELO_ERR_CUDA, "memset");
 
   EstimateParams ep {};
@@ -182,10 +181,13 @@ VeloStatus velo_decode_noalloc(
   ep.module_candidate_num = candidate_num;
   ep.event_estimate = event_estimate;
   ep.bank_index_key = bank_index;
-  ep.designated_stride = (n + 255) / 256;
   ep.status = status;
-  ep.smem_blob_bytes = estimate_blob_bytes;
-  estimate_kernel<<<n, decode_threads, estimate_blob_bytes, stream>>>(ep);
+  ep.list_scratch = reinterpret_cast<uint32_t*>(scratch + off_list);
+  ep.list_capacity = max_clusters;
+  ep.list_alloc = reinterpret_cast<unsigned*>(scratch + off_list_alloc);
+  ep.lists = reinterpret_cast<uint4*>(scratch + off_lists);
+  event_order_kernel<<<event_order_grid(n, true), scan_threads, 0, stream>>>(in, nullptr, bank_index_stride(n), bank_index);
+  estimate_kernel<<<n, decode_threads, 0, stream>>>(ep);
 
   ScanParams sp {};
   sp.jobs[0] = {event_estimate, event_base, n};
@@ -207,10 +209,11 @@ VeloStatus velo_decode_noalloc(
   cp.sorted_container = dev_sorted_velo_cluster_container;
   cp.staging = staging;
   cp.status = status;
-  cp.smem_blob_bytes = cluster_blob_bytes;
+  cp.list_scratch = ep.list_scratch;
+  cp.lists = ep.lists;
   cp.smem_cluster_capacity = cluster_stage_capacity;
   cp.cluster_capacity = static_cast<unsigned>(bound);
-  const unsigned cluster_smem = cluster_sort_blob_offset(cluster_stage_capacity) + cluster_blob_bytes;
+  const unsigned cluster_smem = cluster_sort_smem(cluster_stage_capacity);
   cluster_sort_kernel<decode_threads><<<n, decode_threads, cluster_smem, stream>>>(cp);
   const cudaError_t launch = cudaGetLastError();
   if (launch != cudaSuccess) return fail(VELO_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(launch));

@@ -60,7 +60,7 @@ typedef struct {
 
 /* An event slice in Allen's non-MEP raw-bank layout, on the device. */
 typedef struct {
-  const char* raw;          /* dev_velo_raw_input (16-byte aligned base enables bulk staging) */
+  const char* raw;          /* dev_velo_raw_input */
   const unsigned* offsets;  /* dev_velo_raw_input_offsets [n_events + 1] */
   const unsigned* sizes;    /* dev_velo_raw_input_sizes */
   const unsigned* types;    /* dev_velo_raw_input_types */
@@ -272,9 +272,9 @@ typedef struct {
   unsigned search_threads;
   unsigned search_lanes_per_seed;
   unsigned search_hit_capacity;    /* hits of an event staged in shared memory (15 B each) */
-  unsigned cluster_stage_capacity; /* clusters of an event staged in shared memory (22 B each) */
-  unsigned cluster_blob_bytes;     /* raw event bytes staged by the clustering kernel */
-  unsigned estimate_blob_bytes;    /* raw event bytes staged by the estimate kernel */
+  unsigned cluster_stage_capacity; /* clusters of an event staged in shared memory (22 B each, 64 at least) */
+  unsigned cluster_blob_bytes;     /* accepted within the shared-memory limit, without effect: the decoding */
+  unsigned estimate_blob_bytes;    /* kernels read each raw word once and stage no raw events */
   unsigned persistent;             /* 1: estimate, clustering and search kernels run as many CTAs
                                       as fit the device, claiming events (largest raw size first)
                                       from a work queue; 0: one CTA per event */
