@@ -201,17 +201,28 @@ namespace {
   }
 } // namespace
 
-// search_by_triplet_kernel instantiations (block size, lanes per seed candidate, ring place)
+// search_by_triplet_kernel instantiations (block size, ring place)
 using SearchKernel = void (*)(velo::SearchParams);
 struct SearchVariant {
-  unsigned threads, lanes, ring_global;
+  unsigned threads, ring_global;
   SearchKernel fn;
 };
 static const SearchVariant search_variants[] = {
-#define VELO_SEARCH_VARIANT(T, L, R) {T, L, R, velo::search_by_triplet_kernel<T, L, R>},
+#define VELO_SEARCH_VARIANT(T, R) {T, R, velo::search_by_triplet_kernel<T, R>},
   VELO_SEARCH_CONFIGS(VELO_SEARCH_VARIANT)
 #undef VELO_SEARCH_VARIANT
 };
+
+// The lanes per seed candidate that a launch configuration may name for each block size with the
+// rings in shared memory (with global rings: 0).  They pick no kernel: the seeding gives
+// every candidate the same lanes, with the same results.
+static bool lanes_accepted(unsigned threads, unsigned lanes, unsigned ring_global)
+{
+  if (lanes == 0) return true;
+  if (ring_global) return false;
+  return (threads == 128 && lanes <= 2) || (threads == 256 && (lanes <= 2 || lanes == 4)) ||
+         (threads == 512 && (lanes == 2 || lanes == 4));
+}
 
 // Retina decoding: keys of an event in L2-resident global scratch (shared memory would hold 24 KiB
 // for 3072 keys and allow six CTAs per SM instead of eight), the bucket order of up to 8192
@@ -232,8 +243,9 @@ static SearchKernel gated_search_kernel(unsigned threads, unsigned ring_global)
 
 static const SearchVariant* find_search_variant(unsigned threads, unsigned lanes, unsigned ring_global = 0)
 {
+  if (!lanes_accepted(threads, lanes, ring_global)) return nullptr;
   for (const auto& v : search_variants)
-    if (v.threads == threads && v.lanes == lanes && v.ring_global == ring_global) return &v;
+    if (v.threads == threads && v.ring_global == ring_global) return &v;
   return nullptr;
 }
 
@@ -635,6 +647,7 @@ namespace {
     sp.smem_hit_capacity = c->search_hit_capacity;
     sp.hit_scratch = c->hit_scratch.p;
     sp.ring_scratch = c->ring_scratch.p;
+    sp.used_scratch = c->staging.p; // the clustering's, dead by now
     sp.cluster_capacity = static_cast<unsigned>(c->cap_clusters);
     sp.seed_stats = c->seed_stats.p;
     sp.seed_gate = c->learned ? c->seed_gate.p : nullptr;

@@ -105,6 +105,7 @@ namespace velo {
     unsigned smem_hit_capacity;                   // hits staged in shared memory per event
     unsigned cluster_capacity;                    // allocated T of the containers
     char* hit_scratch;                            // [16 T] staging of events above the capacity
+    char* used_scratch;                           // [24 T] used bits of events above the kernel's shared memory
     uint64_t* ring_scratch;                       // [2048 grid] rings of tracks to follow (RING = 1)
     // learned seed gate (search_by_triplet_gated_kernel): a byte per hit, 0 = the hit is not
     // searched as a seed's middle hit; null = the plain search
@@ -170,18 +171,14 @@ namespace velo {
   __global__ void estimate_kernel(EstimateParams p);
   template<unsigned THREADS> // 128 or 256
   __global__ void cluster_sort_kernel(const __grid_constant__ ClusterSortParams p);
-  template<unsigned THREADS, unsigned LPH, unsigned RING>
-  __global__ void search_by_triplet_kernel(SearchParams p);
-  // flat seeding behind the learned seed gate (and seed-candidate outcome recording);
   // RING = 1: the ring of tracks to follow in global scratch (persistent launches)
+  template<unsigned THREADS, unsigned RING>
+  __global__ void search_by_triplet_kernel(SearchParams p);
+  // the seeding behind the learned seed gate (and seed-candidate outcome recording)
   template<unsigned THREADS, unsigned RING>
   __global__ void search_by_triplet_gated_kernel(SearchParams p);
 #define VELO_GATED_CONFIGS(X) X(128, 0) X(256, 0) X(512, 0) X(128, 1) X(256, 1) X(96, 1) X(64, 1)
-  // (block size, lanes per seed candidate) pairs compiled for the autotuner
-// lanes 0 = flattened seeding (one thread per h1 candidate)
-#define VELO_SEARCH_CONFIGS(X)                                                                                  \
-  X(128, 1, 0) X(128, 2, 0) X(256, 1, 0) X(256, 2, 0) X(256, 4, 0) X(512, 2, 0) X(512, 4, 0) X(128, 0, 0) X(256, 0, 0) \
-    X(512, 0, 0) X(128, 0, 1) X(256, 0, 1) X(96, 0, 1) X(64, 0, 1)
+#define VELO_SEARCH_CONFIGS(X) X(128, 0) X(256, 0) X(512, 0) X(128, 1) X(256, 1) X(96, 1) X(64, 1)
   __global__ void consolidate_kernel(ConsolidateParams p);
   // ---- retina-cluster decoding (VPRetinaCluster banks) ----
   struct RetinaParams {

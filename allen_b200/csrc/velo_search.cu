@@ -6,24 +6,24 @@
 // ThreeHitTracksFilter.cu:48-169.
 //
 // Design.
-//  * The event's sorted hits are staged once as 16-byte records (x, y, z, phi and a flag
-//    byte holding hit_used and the module parity that forwarding needs), so that every
-//    hit a walk visits costs one vector load: in shared memory, or for events above the
+//  * The event's sorted hits are staged once as 16-byte records (x, y, z, phi and the module
+//    parity that forwarding needs), so that every hit a walk visits costs one vector load: in shared memory, or for events above the
 //    shared-memory capacity (and in the tuned launch, every event) in a global scratch
 //    slice that stays in L2, through the same code.
+//  * Which hits are used is a bit per hit in shared memory (the reference's hit_used).
 //  * Within a step every seed candidate (h1) and every track to follow is independent:
-//    seeding only reads hit_used, forwarding only writes it, and each track to follow
-//    owns its track.  Seeding runs LPH lanes per h1: the lanes walk the pendulum of h0
-//    candidates together (ballot), each lane extrapolates its own candidates, and a
-//    shuffle reduction keeps the best (scatter, candidate order) - the same choice as the
-//    reference's sequential loop.  Forwarding runs one thread per track.
+//    seeding only reads the used bits, forwarding only sets them, and each track to follow
+//    owns its track.  Seeding finds the unused h1 by counting bits, a thread each picks its
+//    h0 candidates out of the used bits around h1's phi, then a thread per (h0, h1) extrapolates
+//    and walks the h2 window, and a shuffle reduction keeps the best (scatter, candidate
+//    order) - the same choice as the reference's sequential loop.  Forwarding runs one thread
+//    per track.
 //  * Output slots (ring entries, track numbers, three-hit entries) are assigned by a
 //    block-wide ordered scan in item order, which is the reference's sequential order, so
 //    the track containers come out bit-identical to the reference CPU build.
-//  * The ring of tracks to follow (2048 entries, as the reference) keeps a seed's three
-//    hits in the entry itself; each track's last two hits and hit count live in shared
-//    memory, so forwarding reads no global memory.  Tracks are written to dev_tracks
-//    as they grow.
+//  * An entry of the ring of tracks to follow (2048 entries, as the reference) holds a seed's
+//    three hits, or a track's last two hits, its number and its hit count, so that forwarding
+//    reads nothing else of the track.  Tracks are written to dev_tracks as they grow.
 //  * Leftmost binary searches over a module pair's phi go through a 128-bucket table
 //    per module pair, built once per event, plus a short scan: same index, fewer loads.
 #include <type_traits>
@@ -32,14 +32,21 @@
 
 namespace velo {
 
+  // Ring entries.  Seed: its hits at bits 0, 16, 32.  Track: its last two hits at bits 0 and 16,
+  // its number at bit 32 (one seed at most per hit: 16 bits hold it), its hit count at bit 48.
+  // Both: skipped modules at bit 56, the seed flag at bit 63.
   constexpr uint64_t seed_flag = 1ull << 63;
-  constexpr unsigned skipped_shift = 60;
-  constexpr uint64_t track_number_mask64 = 0x0FFFFFFFull;
-  constexpr unsigned max_tail_tracks = 512; // tracks whose tail lives in shared memory (the others: their container)
-  constexpr uint8_t flag_used = 1;
+  constexpr unsigned skipped_shift = 56;
+  constexpr unsigned skipped_mask = 0x3Fu;
+  constexpr unsigned hits_shift = 48;
   constexpr uint8_t flag_odd_module = 2;
-  constexpr unsigned flat_slots = 1024; // (h1, h0 candidate) slots per chunk of the flat seeding
-  constexpr unsigned pendulum_capacity = 512; // module pairs of up to this many hits get the unused-hit index
+  // Per CTA in shared memory: used bits of an event's first hits (larger events: global scratch),
+  // phi of a module pair's hits (larger pairs: the staged records), ring entries per step
+  constexpr unsigned used_capacity = 8192;
+  constexpr unsigned phi_capacity = 256;
+  constexpr unsigned near_entries = 192;
+  constexpr unsigned seed_window_hits = 256; // hits of the middle module pair that are looked over at once
+  constexpr unsigned seed_slots = 512;       // (h0, h1) doublets in flight
 
   struct ModulePair {
     unsigned hit_start;
@@ -55,47 +62,19 @@ namespace velo {
     // h1 met by the seeding (seed candidates), the candidates whose h0 and h2 windows were
     // searched (the gate let through)
     unsigned local_hits, candidates, searched;
-    uint32_t tail[max_tail_tracks]; // last two hits of a track (hit[n-2] | hit[n-1] << 16)
-    uint8_t tail_n[max_tail_tracks];
-    // bucket tables of the three module pairs a step reads, built one per step
+    uint32_t used[used_capacity / 32 + 1];
+    // bucket tables and phi values of the three module pairs a step reads, filled one per step
     uint16_t bucket[3][n_buckets + 1];
+    int16_t phi[3][phi_capacity];
     // the event's module pairs, last first: a step's three are mps[25 - first] onwards
     ModulePair mps[n_module_pairs];
+    // the seeding's h1, and their h0 candidates in pendulum order (4 or 8 places each)
+    uint16_t seed_h1[seed_slots / 4];
+    uint16_t seed_h0[seed_slots];
   };
-
-  // Shared state of the flat seeding variant: one slot per (h1, candidate order).
-  template<unsigned SLOTS>
-  struct SearchSharedFlatBase : SearchShared {
-    static constexpr unsigned slots = SLOTS;
-    // (h0, h1) doublets of a chunk, packed by pack_doublet(), then overwritten in place
-    // with the best scatter found for the doublet
-    union {
-      uint32_t doublet;
-      float fit;
-    } slot[SLOTS];
-    uint16_t res_h2[SLOTS];
-    // The unused hits of the seeding's previous module pair: how many lie before each
-    // position (the last entry: all of them), and their positions in phi order
-    uint16_t unused_before[pendulum_capacity + 1];
-    uint16_t unused_at[pendulum_capacity];
+  struct SearchSharedGated : SearchShared {
+    uint32_t pass[seed_window_hits / 32]; // the window's unused hits that the gate lets through
   };
-  template<unsigned SLOTS, bool GATED>
-  struct SearchSharedFlatT : SearchSharedFlatBase<SLOTS> {};
-  template<unsigned SLOTS>
-  struct SearchSharedFlatT<SLOTS, true> : SearchSharedFlatBase<SLOTS> {
-    uint16_t cand_list[SLOTS]; // the window's searched candidates (index in the window), h1 order
-  };
-  // flat-seeding kernels: 512 slots for 128 threads (chunks of 64 or 128 h1), which with the
-  // ring in global scratch leaves room for sixteen CTAs per SM
-  template<unsigned THREADS, bool GATED = false>
-  using SearchSharedFlatPlain =
-    SearchSharedFlatT<(THREADS <= 64 ? flat_slots / 4 : (THREADS <= 128 ? flat_slots / 2 : flat_slots)), GATED>;
-
-  // Packed doublet: h0 | h1 index in the chunk << 16 | rank << 25 | (found - 1) << 28
-  __device__ __forceinline__ uint32_t pack_doublet(unsigned h0, unsigned h1_local, unsigned rank, unsigned found)
-  {
-    return h0 | (h1_local << 16) | (rank << 25) | ((found - 1u) << 28);
-  }
 
   // A staged hit, unpacked from its 16-byte record.
   struct Hit {
@@ -116,17 +95,118 @@ namespace velo {
                   (v.w >> 16) & 0xFFu};
     }
     __device__ __forceinline__ int16_t phi(unsigned i) const { return reinterpret_cast<const int16_t*>(r + i)[6]; }
-    __device__ __forceinline__ unsigned flags(unsigned i) const { return reinterpret_cast<const uint8_t*>(r + i)[14]; }
-    __device__ __forceinline__ void mark_used(unsigned i) const { reinterpret_cast<uint8_t*>(r + i)[14] |= flag_used; }
   };
 
-  // Position i < n of the pendulum around p0 in [0, n]: p0, p0 + 1, p0 - 1, p0 + 2, ...
-  // with one wrap (SearchByTriplet.cu:351-370).
-  __device__ __forceinline__ unsigned pendulum(int p0, unsigned i, int n)
+  // The used bits of an event's hits, one word more than they fill.
+  struct UsedBits {
+    uint32_t* w;
+    __device__ __forceinline__ bool operator[](unsigned i) const { return (w[i >> 5] >> (i & 31u)) & 1u; }
+    __device__ __forceinline__ void set(unsigned i) const { atomicOr(w + (i >> 5), 1u << (i & 31u)); }
+    // the unused hits among [i, i + 32) as a word
+    __device__ __forceinline__ uint32_t unused(unsigned i) const
+    {
+      return ~__funnelshift_r(w[i >> 5], w[(i >> 5) + 1], i & 31u);
+    }
+  };
+
+  // The ring of tracks to follow.  A step reads the entries that the step before appended and
+  // appends its own, so only two generations are alive: with NEAR, the first entries of each
+  // lie in shared memory, the others (and without NEAR all of them) in the ring proper.
+  template<bool NEAR>
+  struct Ring {
+    uint64_t* ring;
+    uint64_t* near_ring;  // [2][near_entries]
+    unsigned begin;       // first entry of the generation being appended
+    unsigned parity;      // its half of near_ring
+    __device__ __forceinline__ uint64_t& at(unsigned i, unsigned first, unsigned half) const
+    {
+      if (NEAR && i - first < near_entries) return near_ring[half * near_entries + (i - first)];
+      return ring[i % max_tracks_to_follow];
+    }
+    __device__ __forceinline__ uint64_t& append(unsigned i) const { return at(i, begin, parity); }
+    __device__ __forceinline__ void next_generation(unsigned ttf)
+    {
+      begin = ttf;
+      parity ^= 1u;
+    }
+  };
+
+  // Bits of a word below bit n (n may be 32 or more).
+  __device__ __forceinline__ uint32_t low_bits(uint32_t v, unsigned n) { return n < 32 ? v & ((1u << n) - 1u) : v; }
+
+  // Position of the set bit of rank r (r < popc(v)).
+  __device__ __forceinline__ unsigned select_bit(uint32_t v, unsigned r)
   {
-    const int pos = p0 + ((i & 1u) ? static_cast<int>((i + 1) / 2) : -static_cast<int>(i / 2));
-    return static_cast<unsigned>(pos < 0 ? pos + n : (pos >= n ? pos - n : pos));
+    unsigned at = 0;
+#pragma unroll
+    for (unsigned step = 16; step >= 1; step /= 2) {
+      const unsigned c = __popc(v & ((1u << step) - 1u));
+      if (r >= c) {
+        r -= c;
+        v >>= step;
+        at += step;
+      }
+    }
+    return at;
   }
+
+  // The pendulum around p0 in [0, n] (SearchByTriplet.cu:351-370): step 0 is p0, step 2d - 1 is
+  // p0 + d, step 2d is p0 - d, for steps below n, each position wrapping once.  As offsets from p0
+  // the visit order is 0, +1, -1, +2, ...: two words of unused hits, upwards and downwards from
+  // p0, hold the first 63 steps, and the next candidate is the nearer of their lowest bits (the
+  // upward one first).  Where those hold too few (pairs of more than 62 hits), the walk goes step
+  // by step.
+  struct Pendulum {
+    uint32_t up, down; // bit d: p0 + d; bit d: p0 - 1 - d
+    unsigned k;        // candidates taken
+    __device__ __forceinline__ Pendulum(const UsedBits& used, unsigned start, unsigned n, unsigned p0) : k(0)
+    {
+      const unsigned s = p0 < n ? p0 : 0u;
+      up = low_bits(used.unused(start + s), n - s);
+      if (n - s < 32) up |= used.unused(start) << (n - s);
+      up = low_bits(up, n / 2 + 1);
+      if (s >= 32) {
+        down = __brev(used.unused(start + s - 32));
+      }
+      else {
+        const uint32_t end = n >= 32 ? used.unused(start + n - 32) : used.unused(start) << (32 - n);
+        down = __brev(end) << s;
+        if (s > 0) down |= __brev(used.unused(start) << (32 - s));
+      }
+      down = low_bits(down, min((n - 1) / 2, 31u));
+    }
+    // The next candidate's position; there is one (the caller knows the number of unused hits).
+    __device__ __forceinline__ unsigned next(const UsedBits& used, unsigned start, unsigned n, unsigned p0)
+    {
+      if ((up | down) == 0) {
+        unsigned found = 0;
+        for (unsigned i = 0;; ++i) {
+          const unsigned pos = wrap(int(p0) + ((i & 1u) ? int((i + 1) / 2) : -int(i / 2)), n);
+          if (i >= n || (!used[start + pos] && found++ == k)) {
+            ++k;
+            return pos;
+          }
+        }
+      }
+      ++k;
+      const int u = up ? __ffs(up) - 1 : 64;
+      const int d = down ? __ffs(down) : 64;
+      int offset;
+      if (u <= d) {
+        offset = u;
+        up &= up - 1;
+      }
+      else {
+        offset = -d;
+        down &= down - 1;
+      }
+      return wrap(int(p0) + offset, n);
+    }
+    static __device__ __forceinline__ unsigned wrap(int pos, unsigned n)
+    {
+      return static_cast<unsigned>(pos < 0 ? pos + int(n) : (pos >= int(n) ? pos - int(n) : pos));
+    }
+  };
 
   // The first h2 of the circular window walk: start % n (0 for an empty module pair), without
   // a division for start in [0, n], leftmost()'s range.
@@ -136,12 +216,18 @@ namespace velo {
     return x < n ? x : (x == n || n == 0 ? 0u : x % n);
   }
 
-  // leftmost() over the staged hits [start, start + n) of a module pair.
-  __device__ __forceinline__ int leftmost_hit(const uint16_t* table, const Hits& h, unsigned start, unsigned n, int16_t value)
+  // leftmost() over a module pair's hits, through the phi values of its table slot when they fit.
+  __device__ __forceinline__ int leftmost_hit(const SearchShared& s, const Hits& h, const ModulePair& m, int16_t value)
   {
-    unsigned i = table[bucket_of(value)];
-    while (i < n && h.phi(start + i) < value)
-      ++i;
+    unsigned i = s.bucket[m.table][bucket_of(value)];
+    if (m.hit_num <= phi_capacity) {
+      while (i < m.hit_num && s.phi[m.table][i] < value)
+        ++i;
+    }
+    else {
+      while (i < m.hit_num && h.phi(m.hit_start + i) < value)
+        ++i;
+    }
     return static_cast<int>(i);
   }
 
@@ -182,21 +268,8 @@ namespace velo {
     return before + incl - v;
   }
 
-  // Block-wide exclusive scan of v (every thread of the block calls it).
-  __device__ __forceinline__ unsigned scan1(SearchShared& s, Counters& c, unsigned v, unsigned& total)
-  {
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= static_cast<unsigned>(o)) incl += t;
-    }
-    return scan_block(s, c, incl, v, total);
-  }
-
-  // scan1() of up to three 0/1 flags packed at bits 0, S1 and S2 (each field wide enough for
-  // a block total), the warp part by ballots.
+  // Block-wide exclusive scan of up to three 0/1 flags packed at bits 0, S1 and S2 (each field
+  // wide enough for a block total), the warp part by ballots.
   template<unsigned NF, unsigned S1 = 16, unsigned S2 = 32>
   __device__ __forceinline__ unsigned scan_flags(SearchShared& s, Counters& c, bool f0, bool f1, bool f2, unsigned& total)
   {
@@ -245,355 +318,176 @@ namespace velo {
     x.phi = hit_phi_16(k, xp, yp);
     const int16_t lo = static_cast<int16_t>(x.phi - static_cast<int16_t>(k.phi_tolerance_i16));
     // find_forward_candidate returns the index as int16
-    x.start = static_cast<int16_t>(leftmost_hit(s.bucket[next.table], h, next.hit_start, next.hit_num, lo));
+    x.start = static_cast<int16_t>(leftmost_hit(s, h, next, lo));
     return x;
   }
 
-  // One h0 candidate of a seed (SearchByTriplet.cu:374-432): updates (best_fit, best_c,
-  // best_h0, best_h2) with strict improvement, in window order.
-  __device__ __forceinline__ void seed_candidate(
-    const Constants& k,
-    const SearchShared& s,
-    const Hits& h,
-    const ModulePair& prev,
-    const ModulePair& next,
-    float h1x,
-    float h1y,
-    float h1z,
-    unsigned h0,
-    unsigned c,
-    float& best_fit,
-    unsigned& best_c,
-    unsigned& best_h0,
-    unsigned& best_h2)
-  {
-    const int16_t tol = static_cast<int16_t>(k.phi_tolerance_i16);
-    const Hit a = h[h0];
-    const float h0x = a.x, h0y = a.y, h0z = a.z;
-    const float td = __fdiv_rn(1.0f, h1z - h0z);
-    const float txn = h1x - h0x;
-    const float tyn = h1y - h0y;
-    const float tx = txn * td;
-    const float ty = tyn * td;
-    const Extrapolation f = extrapolate(k, s, h, next, h0x, h0y, tx, ty, next.z[0] - prev.z[0]);
-    // circular walk from the candidate: index (start + j) % n without a division per step
-    unsigned idx = first_candidate(f.start, next.hit_num);
-    for (unsigned j = 0; j < next.hit_num; ++j, idx = (idx + 1 == next.hit_num) ? 0u : idx + 1) {
-      const unsigned h2 = next.hit_start + idx;
-      const Hit b = h[h2];
-      if (phi_outside(b.phi, f.phi, tol)) break;
-      if (b.flags & flag_used) continue;
-      const float dz = b.z - h0z;
-      const float predx = h0x + tx * dz;
-      const float predy = h0y + ty * dz;
-      const float dx = predx - b.x;
-      const float dy = predy - b.y;
-      const float scatter = dx * dx + dy * dy;
-      if (scatter < best_fit) {
-        best_fit = scatter;
-        best_c = c;
-        best_h0 = h0;
-        best_h2 = h2;
-      }
-    }
-  }
-
-  // Seeding over the current module pair (SearchByTriplet.cu:298-446), LPH lanes per h1.
-  template<unsigned LPH>
-  __device__ __forceinline__ void seeding(
-    SearchShared& s, uint64_t* ring, Counters& cnt, const Constants& k, const Hits& h, const ModulePair* md,
-    unsigned n_candidates)
-  {
-    const ModulePair &prev = md[0], &cur = md[1], &next = md[2];
-    const unsigned groups = blockDim.x / LPH;
-    const unsigned g = threadIdx.x / LPH;
-    const unsigned l = threadIdx.x % LPH;
-    const unsigned lane0 = (threadIdx.x & 31u) & ~(LPH - 1);
-    const unsigned gmask = (LPH == 32 ? 0xFFFFFFFFu : ((1u << LPH) - 1u)) << lane0;
-    for (unsigned c0 = 0; c0 < cur.hit_num; c0 += groups) {
-      const unsigned r = c0 + g;
-      const unsigned h1 = cur.hit_start + r;
-      const bool valid = r < cur.hit_num && !(h.flags(h1) & flag_used);
-      float best_fit = k.max_scatter;
-      unsigned best_c = 0xFFFFFFFFu, best_h0 = 0, best_h2 = 0;
-      if (valid) {
-        const Hit b = h[h1];
-        const float h1x = b.x, h1y = b.y, h1z = b.z;
-        const int p0 = leftmost_hit(s.bucket[prev.table], h, prev.hit_start, prev.hit_num, b.phi);
-        const int n_prev = static_cast<int>(prev.hit_num);
-        unsigned found = 0;
-        for (unsigned i0 = 0; i0 < prev.hit_num && found < n_candidates; i0 += LPH) {
-          const unsigned i = i0 + l;
-          bool ok = false;
-          unsigned h0 = 0;
-          if (i < prev.hit_num) {
-            // pendulum p0, p0 + 1, p0 - 1, p0 + 2, ... with one wrap (SearchByTriplet.cu:351-370)
-            const int pos = p0 + ((i & 1u) ? static_cast<int>((i + 1) / 2) : -static_cast<int>(i / 2));
-            const int in_bounds = pos < 0 ? pos + n_prev : (pos >= n_prev ? pos - n_prev : pos);
-            h0 = prev.hit_start + static_cast<unsigned>(in_bounds);
-            ok = !(h.flags(h0) & flag_used);
-          }
-          const unsigned ballot = (__ballot_sync(gmask, ok) & gmask) >> lane0;
-          const unsigned rank = __popc(ballot & ((1u << l) - 1u));
-          if (ok && found + rank < n_candidates) {
-            seed_candidate(k, s, h, prev, next, h1x, h1y, h1z, h0, found + rank, best_fit, best_c, best_h0, best_h2);
-          }
-          found += __popc(ballot);
-        }
-#pragma unroll
-        for (unsigned o = LPH / 2; o >= 1; o /= 2) {
-          const float of = __shfl_xor_sync(gmask, best_fit, o);
-          const unsigned oc = __shfl_xor_sync(gmask, best_c, o);
-          const unsigned o0 = __shfl_xor_sync(gmask, best_h0, o);
-          const unsigned o2 = __shfl_xor_sync(gmask, best_h2, o);
-          if (of < best_fit || (of == best_fit && oc < best_c)) {
-            best_fit = of;
-            best_c = oc;
-            best_h0 = o0;
-            best_h2 = o2;
-          }
-        }
-      }
-      const bool ok = valid && l == 0 && best_fit < k.max_scatter;
-      const unsigned unused = (valid && l == 0) ? 1u : 0u;
-      unsigned total;
-      const unsigned excl = scan_flags<2>(s, cnt, ok, unused != 0, false, total);
-      if (ok) {
-        const unsigned tn = (cnt.ttf + (excl & 0xFFFFu)) % max_tracks_to_follow;
-        ring[tn] = seed_flag | (uint64_t(best_h0 & 0xFFFFu)) | (uint64_t(h1 & 0xFFFFu) << 16) |
-                     (uint64_t(best_h2 & 0xFFFFu) << 32);
-      }
-      cnt.ttf += total & 0xFFFFu;
-      if (threadIdx.x == 0) s.local_hits += total >> 16;
-    }
-  }
-
-  __device__ __forceinline__ unsigned candidate_h0(uint64_t lo, uint64_t hi, unsigned c)
-  {
-    return static_cast<unsigned>((c < 4 ? lo >> (16 * c) : hi >> (16 * (c - 4))) & 0xFFFFu);
-  }
-
-  // Seeding with the candidates flattened (SearchByTriplet.cu:298-446).  The window's unused
-  // h1 are first compacted to threads 0, 1, ... in h1 order.  Phase A, one thread per h1,
-  // walks the pendulum and keeps its first n_candidates unused h0 in registers; a block scan
-  // packs all (h0, h1) doublets of the chunk into one list.
-  // Phase B, one thread per doublet, extrapolates and scans the h2 window.  Phase C, one
-  // thread per h1, keeps the first strictly best of its doublets in candidate order (the
-  // reference's sequential choice) and queues the seed in h1 order.  Phase B runs the same
-  // path on every lane and has no idle slots for h1 with fewer than n_candidates doublets.
+  // Seeding over the current module pair (SearchByTriplet.cu:298-446).  Phase A, one thread per
+  // unused h1: its rank among the window's unused hits names it (a word of bits per lane and a
+  // bisection over their counts), and the pendulum its h0 candidates; every h1 has the same
+  // number of them, the unused hits of the previous module pair or n_candidates.  Phase B, one
+  // thread per (h0, h1) doublet: the h2 window; the doublets of an h1 are neighbouring lanes,
+  // whose shuffle reduction keeps the best (scatter, candidate order), the reference's
+  // sequential choice, and a scan queues the seeds in h1 order.  Two barriers per chunk.
   // GATED kernels take the learned seed gate (gate, event-relative, or null): an unused h1
   // whose gate byte is 0 is not searched; and, for training, record each unused h1's
   // outcome (outcome: 1 no seed, 2 seed; null = off).
-  template<bool GATED, typename Flat>
-  __device__ __forceinline__ void seeding_flat(
-    Flat& s,
-    uint64_t* ring,
+  template<bool GATED, typename Shared, typename RingT>
+  __device__ __forceinline__ void seeding(
+    Shared& s,
+    const RingT& ring,
     Counters& cnt,
     const Constants& k,
     const Hits& h,
+    const UsedBits& used,
     const ModulePair* md,
     unsigned n_candidates,
     const uint8_t* gate,
     uint8_t* outcome)
   {
     const ModulePair &prev = md[0], &cur = md[1], &next = md[2];
-    const unsigned per_chunk = min(blockDim.x, Flat::slots / n_candidates);
-    const int n_prev = static_cast<int>(prev.hit_num);
+    const unsigned lane = threadIdx.x & 31u;
     const int16_t tol = static_cast<int16_t>(k.phi_tolerance_i16);
-    // The unused-hit index of the previous module pair (its used flags do not change
-    // during the seeding), when a module pair has hits to seed and fits the index
-    const bool indexed = cur.hit_num > 0 && prev.hit_num <= pendulum_capacity;
-    unsigned n_unused = 0;
-    if (indexed) {
-      for (unsigned i0 = 0; i0 < prev.hit_num; i0 += blockDim.x) {
-        const unsigned i = i0 + threadIdx.x;
-        const bool unused = i < prev.hit_num && !(h.flags(prev.hit_start + i) & flag_used);
-        unsigned total;
-        const unsigned before = n_unused + scan_flags<1>(s, cnt, unused, false, false, total);
-        if (i < prev.hit_num) s.unused_before[i] = static_cast<uint16_t>(before);
-        if (unused) s.unused_at[before] = static_cast<uint16_t>(i);
-        n_unused += total;
-      }
-      if (threadIdx.x == 0) s.unused_before[prev.hit_num] = static_cast<uint16_t>(n_unused);
-      __syncthreads();
-    }
-    for (unsigned c0 = 0; c0 < cur.hit_num; c0 += per_chunk) {
-      const unsigned n_h1 = min(per_chunk, cur.hit_num - c0);
-      // Gated: the window's candidates compacted in h1 order (its unused hits that the gate
-      // lets through, one per thread from thread 0 on), so that the phases below run on as
-      // few warps as there are candidates.  Plain: thread i takes the window's hit i (the
-      // compaction's scan and barrier cost the plain search more than they save).
-      bool searched;
-      unsigned hl;
+    // the unused hits of the previous module pair
+    unsigned n_h0 = 0;
+    for (unsigned i = 32 * lane; i < prev.hit_num; i += 1024)
+      n_h0 += __popc(low_bits(used.unused(prev.hit_start + i), prev.hit_num - i));
+    n_h0 = min(__reduce_add_sync(0xFFFFFFFFu, n_h0), n_candidates);
+    const unsigned places_log = n_candidates > 4 ? 3 : 2;
+    for (unsigned w0 = 0; w0 < cur.hit_num; w0 += seed_window_hits) {
+      const unsigned n_window = min(seed_window_hits, cur.hit_num - w0);
+      const unsigned first = cur.hit_start + w0;
+      // the window's unused hits, 32 per lane of every warp
+      uint32_t word = 32 * lane < n_window ? low_bits(used.unused(first + 32 * lane), n_window - 32 * lane) : 0u;
       if constexpr (GATED) {
-        unsigned n_searched;
-        {
-          const unsigned hw = cur.hit_start + c0 + threadIdx.x;
-          const bool valid = threadIdx.x < n_h1 && !(h.flags(hw) & flag_used);
-          const bool pass = valid && (gate == nullptr || gate[hw] != 0);
-          unsigned total;
-          const unsigned excl = scan_flags<2>(s, cnt, pass, valid, false, total);
-          if (pass) s.cand_list[excl & 0xFFFFu] = static_cast<uint16_t>(threadIdx.x);
-          n_searched = total & 0xFFFFu;
-          if (threadIdx.x == 0) {
-            s.local_hits += total >> 16;
-            s.candidates += total >> 16;
-            s.searched += n_searched;
-          }
+        const unsigned unused = __reduce_add_sync(0xFFFFFFFFu, __popc(word));
+        if (threadIdx.x == 0) {
+          s.local_hits += unused;
+          s.candidates += unused;
         }
-        __syncthreads();
-        searched = threadIdx.x < n_searched;
-        hl = searched ? s.cand_list[threadIdx.x] : 0u;
-      }
-      else {
-        hl = threadIdx.x;
-        searched = threadIdx.x < n_h1 && !(h.flags(cur.hit_start + c0 + hl) & flag_used);
-      }
-      const unsigned h1 = cur.hit_start + c0 + hl;
-      // Phase A: candidates c < 4 in the 16-bit fields of cand_lo, 4..7 in cand_hi, the first
-      // n_candidates unused h0 of the pendulum p0, p0 + 1, p0 - 1, p0 + 2, ... (one wrap).
-      // With the unused-hit index, the pendulum's unused hits are the merge of the index's
-      // run from p0 upwards (pendulum step 2d - 1 at offset d > 0, 0 at p0) and its run below
-      // p0 (step 2d at offset d), each wrapping once, taken while the step is below n.
-      uint64_t cand_lo = 0, cand_hi = 0;
-      unsigned found = 0;
-      if (searched) {
-        const int p0 = leftmost_hit(s.bucket[prev.table], h, prev.hit_start, prev.hit_num, h.phi(h1));
-        if (indexed) {
-          const int u = static_cast<int>(n_unused);
-          const int r = s.unused_before[p0];
-          // step and position of the k-th unused hit upwards (k >= r) and downwards (k < r)
-          auto up = [&](int kk, unsigned& pos) {
-            if (kk >= 2 * u) return static_cast<unsigned>(n_prev);
-            const int q = s.unused_at[kk < u ? kk : kk - u];
-            pos = static_cast<unsigned>(q);
-            const int d = (kk < u ? q : q + n_prev) - p0;
-            return d == 0 ? 0u : static_cast<unsigned>(2 * d - 1);
-          };
-          auto down = [&](int kk, unsigned& pos) {
-            if (kk < -u) return static_cast<unsigned>(n_prev);
-            const int q = s.unused_at[kk >= 0 ? kk : kk + u];
-            pos = static_cast<unsigned>(q);
-            return static_cast<unsigned>(2 * (p0 - (kk >= 0 ? q : q - n_prev)));
-          };
-          int ku = r, kd = r - 1;
-          unsigned pu = 0, pd = 0;
-          unsigned iu = up(ku, pu), id = down(kd, pd);
-          while (found < n_candidates) {
-            const bool upward = iu < id;
-            if ((upward ? iu : id) >= prev.hit_num) break;
-            const unsigned h0 = prev.hit_start + (upward ? pu : pd);
-            if (found < 4) cand_lo |= uint64_t(h0) << (16 * found);
-            else cand_hi |= uint64_t(h0) << (16 * (found - 4));
-            ++found;
-            if (upward) iu = up(++ku, pu);
-            else id = down(--kd, pd);
+        if (gate != nullptr) {
+          for (unsigned i = threadIdx.x; i < (n_window + 31u) / 32u * 32u; i += blockDim.x) {
+            const uint32_t pass = __ballot_sync(0xFFFFFFFFu, i < n_window && !used[first + i] && gate[first + i] != 0);
+            if (lane == 0) s.pass[i / 32] = pass;
           }
+          __syncthreads();
+          word = 32 * lane < n_window ? s.pass[lane] : 0u;
         }
-        else {
-          for (unsigned i = 0; i < prev.hit_num && found < n_candidates; ++i) {
-            const unsigned h0 = prev.hit_start + pendulum(p0, i, n_prev);
-            if (!(h.flags(h0) & flag_used)) {
-              if (found < 4) cand_lo |= uint64_t(h0) << (16 * found);
-              else cand_hi |= uint64_t(h0) << (16 * (found - 4));
-              ++found;
+      }
+      static_assert(seed_window_hits == 256, "the scan and the bisection are over 8 words");
+      unsigned before = __popc(word); // the hits up to this lane's word, then those before it
+#pragma unroll
+      for (unsigned o = 1; o < 8; o *= 2) {
+        const unsigned t = __shfl_up_sync(0xFFFFFFFFu, before, o);
+        if (lane >= o) before += t;
+      }
+      const unsigned n_h1 = __shfl_sync(0xFFFFFFFFu, before, 7);
+      before -= __popc(word);
+      const unsigned per_chunk = min(blockDim.x, seed_slots >> places_log);
+      for (unsigned c0 = 0; c0 < n_h1; c0 += per_chunk) {
+        const unsigned n_chunk = min(per_chunk, n_h1 - c0);
+        // Phase A
+        if ((threadIdx.x & ~31u) < n_chunk) { // warps with work, whole
+          const unsigned rank = c0 + min(threadIdx.x, n_chunk - 1);
+          unsigned at = 0; // the last word with no more than rank hits before it
+#pragma unroll
+          for (unsigned step = 4; step >= 1; step /= 2)
+            if (__shfl_sync(0xFFFFFFFFu, before, at + step) <= rank) at += step;
+          const uint32_t bits = __shfl_sync(0xFFFFFFFFu, word, at);
+          const unsigned offset = rank - __shfl_sync(0xFFFFFFFFu, before, at);
+          if (threadIdx.x < n_chunk) {
+            const unsigned h1 = first + 32 * at + select_bit(bits, offset);
+            s.seed_h1[threadIdx.x] = static_cast<uint16_t>(h1);
+            if (n_h0 > 0) {
+              const unsigned p0 = static_cast<unsigned>(leftmost_hit(s, h, prev, h.phi(h1)));
+              Pendulum pendulum(used, prev.hit_start, prev.hit_num, p0);
+              for (unsigned c = 0; c < n_h0; ++c)
+                s.seed_h0[(threadIdx.x << places_log) + c] =
+                  static_cast<uint16_t>(prev.hit_start + pendulum.next(used, prev.hit_start, prev.hit_num, p0));
             }
           }
         }
-      }
-      unsigned n_doublets;
-      const unsigned first = scan1(s, cnt, found, n_doublets);
-      for (unsigned c = 0; c < found; ++c)
-        s.slot[first + c].doublet = pack_doublet(candidate_h0(cand_lo, cand_hi, c), hl, c, found);
-      __syncthreads();
-      // keep_mask bit c: doublet c's slot in the packed list (every doublet is scanned)
-      const unsigned keep_mask = (1u << found) - 1u;
-      // Phase B
-      for (unsigned q = threadIdx.x; q < n_doublets; q += blockDim.x) {
-        const uint32_t d = s.slot[q].doublet;
-        const unsigned h0 = d & 0xFFFFu;
-        const unsigned hh1 = cur.hit_start + c0 + ((d >> 16) & 0x1FFu);
-        float best_fit = k.max_scatter;
-        unsigned best_h2 = 0xFFFFu;
-        const Hit a = h[h0], b = h[hh1];
-        const float h1x = b.x, h1y = b.y, h1z = b.z;
-        const float h0x = a.x, h0y = a.y, h0z = a.z;
-        const float td = __fdiv_rn(1.0f, h1z - h0z);
-        const float txn = h1x - h0x;
-        const float tyn = h1y - h0y;
-        const float tx = txn * td;
-        const float ty = tyn * td;
-        const Extrapolation f = extrapolate(k, s, h, next, h0x, h0y, tx, ty, next.z[0] - prev.z[0]);
-        unsigned idx = first_candidate(f.start, next.hit_num);
-        for (unsigned j = 0; j < next.hit_num; ++j, idx = (idx + 1 == next.hit_num) ? 0u : idx + 1) {
-          const unsigned h2 = next.hit_start + idx;
-          const Hit c = h[h2];
-          if (phi_outside(c.phi, f.phi, tol)) break;
-          if (c.flags & flag_used) continue;
-          const float dz = c.z - h0z;
-          const float predx = h0x + tx * dz;
-          const float predy = h0y + ty * dz;
-          const float dx = predx - c.x;
-          const float dy = predy - c.y;
-          const float scatter = dx * dx + dy * dy;
-          if (scatter < best_fit) {
-            best_fit = scatter;
-            best_h2 = h2;
+        __syncthreads();
+        // Phase B
+        for (unsigned q0 = 0; q0 < n_chunk << places_log; q0 += blockDim.x) {
+          const unsigned q = q0 + threadIdx.x, i = q >> places_log, c = q & ((1u << places_log) - 1u);
+          float best_fit = k.max_scatter;
+          unsigned best = 0, best_c = c; // best: h0 | h2 << 16
+          unsigned h1 = 0;
+          if (i < n_chunk && c < n_h0) {
+            h1 = s.seed_h1[i];
+            const unsigned h0 = s.seed_h0[q];
+            const Hit a = h[h0], b = h[h1];
+            const float td = __frcp_rn(b.z - a.z);
+            const float tx = (b.x - a.x) * td;
+            const float ty = (b.y - a.y) * td;
+            const Extrapolation f = extrapolate(k, s, h, next, a.x, a.y, tx, ty, next.z[0] - prev.z[0]);
+            // circular walk from the candidate: index (start + j) % n without a division per step
+            unsigned idx = first_candidate(f.start, next.hit_num);
+            for (unsigned j = 0; j < next.hit_num; ++j, idx = (idx + 1 == next.hit_num) ? 0u : idx + 1) {
+              const unsigned h2 = next.hit_start + idx;
+              const Hit d = h[h2];
+              if (phi_outside(d.phi, f.phi, tol)) break;
+              const float dz = d.z - a.z;
+              const float dx = (a.x + tx * dz) - d.x;
+              const float dy = (a.y + ty * dz) - d.y;
+              const float scatter = dx * dx + dy * dy;
+              if (scatter < best_fit && !used[h2]) {
+                best_fit = scatter;
+                best = h0 | (h2 << 16);
+              }
+            }
           }
-        }
-        s.slot[q].fit = best_fit;
-        s.res_h2[q] = static_cast<uint16_t>(best_h2);
-      }
-      __syncthreads();
-      // Phase C
-      bool ok = false;
-      unsigned best_h0 = 0, best_h2 = 0, best_c = 0xFFFFFFFFu;
-      if (searched) {
-        float best_fit = k.max_scatter;
-        unsigned at = first;
-        for (unsigned c = 0; c < found; ++c) {
-          if (!(keep_mask & (1u << c))) continue;
-          const float fit = s.slot[at].fit;
-          if (fit < best_fit) {
-            best_fit = fit;
-            best_c = c;
-            best_h0 = candidate_h0(cand_lo, cand_hi, c);
-            best_h2 = s.res_h2[at];
+          for (unsigned o = 1; o < 1u << places_log; o *= 2) {
+            const float of = __shfl_xor_sync(0xFFFFFFFFu, best_fit, o);
+            const unsigned oc = __shfl_xor_sync(0xFFFFFFFFu, best_c, o);
+            const unsigned ob = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+            if (of < best_fit || (of == best_fit && oc < best_c)) {
+              best_fit = of;
+              best_c = oc;
+              best = ob;
+            }
           }
-          ++at;
+          const bool first_lane = c == 0 && i < n_chunk;
+          const bool ok = first_lane && best_fit < k.max_scatter;
+          if (GATED && outcome != nullptr && first_lane) outcome[s.seed_h1[i]] = ok ? 2 : 1;
+          unsigned n_seeds;
+          const unsigned excl = scan_flags<1>(s, cnt, ok, false, false, n_seeds);
+          if (ok) {
+            ring.append(cnt.ttf + excl) =
+              seed_flag | uint64_t(best & 0xFFFFu) | (uint64_t(h1 & 0xFFFFu) << 16) | (uint64_t(best >> 16) << 32);
+          }
+          cnt.ttf += n_seeds;
         }
-        ok = best_fit < k.max_scatter;
-        if (GATED && outcome != nullptr) outcome[h1] = ok ? 2 : 1;
       }
-      unsigned total;
-      const unsigned excl = scan_flags<GATED ? 1 : 2>(s, cnt, ok, !GATED && searched, false, total);
-      if (ok) {
-        const unsigned tn = (cnt.ttf + (excl & 0xFFFFu)) % max_tracks_to_follow;
-        ring[tn] = seed_flag | (uint64_t(best_h0 & 0xFFFFu)) | (uint64_t(h1 & 0xFFFFu) << 16) |
-                     (uint64_t(best_h2 & 0xFFFFu) << 32);
+      if (threadIdx.x == 0) {
+        if (!GATED) {
+          s.local_hits += n_h1;
+          s.candidates += n_h1;
+        }
+        s.searched += n_h1;
       }
-      cnt.ttf += total & 0xFFFFu;
-      if (!GATED && threadIdx.x == 0) {
-        s.local_hits += total >> 16;
-        s.candidates += total >> 16;
-        s.searched += total >> 16;
-      }
+      if (GATED && gate != nullptr && w0 + seed_window_hits < cur.hit_num) __syncthreads(); // s.pass is read
     }
   }
 
-  // Forwarding of the tracks to follow (SearchByTriplet.cu:451-609), one thread per track.
+  // Forwarding of the tracks to follow (SearchByTriplet.cu:451-609), one thread per track.  The
+  // hits the >= 4 hit tracks gained are added to the thread's track_hits.
+  template<typename Shared, typename RingT>
   __device__ __forceinline__ void forwarding(
-    SearchShared& s,
-    uint64_t* ring,
+    Shared& s,
+    const RingT& ring,
     Counters& cnt,
     const Constants& k,
     const Hits& h,
+    const UsedBits& used,
     const ModulePair& next,
     unsigned prev_ttf,
     unsigned diff_ttf,
     TrackHits* tracks,
     unsigned track_limit,
     TrackletHits* three_hit,
+    unsigned& track_hits,
     unsigned* status)
   {
     const int16_t tol = static_cast<int16_t>(k.phi_tolerance_i16);
@@ -601,55 +495,30 @@ namespace velo {
       const unsigned kk = c0 + threadIdx.x;
       const bool active = kk < diff_ttf;
       uint64_t entry = 0;
-      unsigned nh = 0, tn = 0, h0n = 0, h1n = 0;
+      unsigned h0n = 0, h1n = 0;
       bool is_seed = false, found = false;
       unsigned best_h2 = 0;
       if (active) {
-        entry = ring[(prev_ttf + kk) % max_tracks_to_follow];
+        entry = ring.at(prev_ttf + kk, prev_ttf, ring.parity ^ 1u);
         is_seed = (entry & seed_flag) != 0;
-        if (is_seed) {
-          nh = 3;
-          h0n = static_cast<unsigned>(entry >> 16) & 0xFFFFu;
-          h1n = static_cast<unsigned>(entry >> 32) & 0xFFFFu;
-        }
-        else {
-          tn = static_cast<unsigned>(entry & track_number_mask64);
-          if (tn < max_tail_tracks) {
-            nh = s.tail_n[tn];
-            h0n = s.tail[tn] & 0xFFFFu;
-            h1n = s.tail[tn] >> 16;
-          }
-          else if (tn < track_limit) {
-            nh = tracks[tn].hits_num;
-            if (nh < 2 || nh > max_track_size) nh = 2;
-            h0n = tracks[tn].hits[nh - 2];
-            h1n = tracks[tn].hits[nh - 1];
-          }
-          else {
-            nh = 3; // a track that did not fit its container, flagged when created
-          }
-        }
+        const unsigned pair = static_cast<unsigned>(is_seed ? entry >> 16 : entry);
+        h0n = pair & 0xFFFFu;
+        h1n = pair >> 16;
         const Hit a = h[h0n], b = h[h1n];
-        const float h0x = a.x, h0y = a.y, h0z = a.z;
         const unsigned odd = (a.flags & flag_odd_module) ? 1u : 0u;
-        const float h1x = b.x, h1y = b.y, h1z = b.z;
-        const float td = __fdiv_rn(1.0f, h1z - h0z);
-        const float txn = h1x - h0x;
-        const float tyn = h1y - h0y;
-        const float tx = txn * td;
-        const float ty = tyn * td;
+        const float td = __frcp_rn(b.z - a.z);
+        const float tx = (b.x - a.x) * td;
+        const float ty = (b.y - a.y) * td;
         float best_fit = k.max_scatter;
-        const Extrapolation f = extrapolate(k, s, h, next, h0x, h0y, tx, ty, next.z[odd] - h0z);
+        const Extrapolation f = extrapolate(k, s, h, next, a.x, a.y, tx, ty, next.z[odd] - a.z);
         unsigned idx = first_candidate(f.start, next.hit_num);
         for (unsigned j = 0; j < next.hit_num; ++j, idx = (idx + 1 == next.hit_num) ? 0u : idx + 1) {
           const unsigned h2 = next.hit_start + idx;
           const Hit c = h[h2];
           if (phi_outside(c.phi, f.phi, tol)) break;
-          const float dz = c.z - h0z;
-          const float predx = h0x + tx * dz;
-          const float predy = h0y + ty * dz;
-          const float dx = predx - c.x;
-          const float dy = predy - c.y;
+          const float dz = c.z - a.z;
+          const float dx = (a.x + tx * dz) - c.x;
+          const float dy = (a.y + ty * dz) - c.y;
           const float scatter = dx * dx + dy * dy;
           if (scatter < best_fit) {
             best_fit = scatter;
@@ -658,23 +527,24 @@ namespace velo {
           }
         }
       }
-      const unsigned skipped = static_cast<unsigned>(entry >> skipped_shift) & 0x7u;
+      const unsigned nh = is_seed ? 3u : static_cast<unsigned>(entry >> hits_shift) & 0x1Fu;
+      const unsigned skipped = static_cast<unsigned>(entry >> skipped_shift) & skipped_mask;
       const bool new_track = active && found && is_seed;
       const bool enqueue =
         active && ((found && nh + 1 < max_track_size) || (!found && skipped < k.max_skipped_modules));
-      const bool three = active && !found && !(skipped < k.max_skipped_modules) && nh == 3 && is_seed;
+      const bool three = active && !found && !(skipped < k.max_skipped_modules) && is_seed;
       unsigned total;
       const unsigned excl =
         scan_flags<3, 10, 20>(s, cnt, new_track, enqueue, three, total);
       if (active) {
-        unsigned track_number = tn;
         if (found) {
-          h.mark_used(best_h2);
+          used.set(best_h2);
+          unsigned track_number = static_cast<unsigned>(entry >> 32) & 0xFFFFu;
           if (is_seed) {
             const unsigned t0 = static_cast<unsigned>(entry) & 0xFFFFu;
-            h.mark_used(t0);
-            h.mark_used(h0n);
-            h.mark_used(h1n);
+            used.set(t0);
+            used.set(h0n);
+            used.set(h1n);
             track_number = cnt.n_tracks + (excl & 0x3FFu);
             if (track_number < track_limit) {
               TrackHits& t = tracks[track_number];
@@ -687,30 +557,21 @@ namespace velo {
             else {
               set_error(status, err_track_capacity);
             }
-            if (track_number < max_tail_tracks) {
-              s.tail[track_number] = h1n | (best_h2 << 16);
-              s.tail_n[track_number] = 4;
-            }
           }
-          else {
-            if (tn < track_limit) {
-              tracks[tn].hits[nh] = static_cast<uint16_t>(best_h2);
-              tracks[tn].hits_num = static_cast<uint8_t>(nh + 1);
-            }
-            if (tn < max_tail_tracks) {
-              s.tail[tn] = h1n | (best_h2 << 16);
-              s.tail_n[tn] = static_cast<uint8_t>(nh + 1);
-            }
+          else if (track_number < track_limit) {
+            tracks[track_number].hits[nh] = static_cast<uint16_t>(best_h2);
+            tracks[track_number].hits_num = static_cast<uint8_t>(nh + 1);
           }
-          atomicAdd(&s.track_hits, is_seed ? 4u : 1u);
+          track_hits += is_seed ? 4u : 1u;
+          entry = uint64_t(h1n) | (uint64_t(best_h2 & 0xFFFFu) << 16) | (uint64_t(track_number & 0xFFFFu) << 32) |
+                  (uint64_t(nh + 1) << hits_shift);
         }
-        if (enqueue) {
-          // requeued entries keep the seed's hits or the track number, with skipped + 1
-          const uint64_t value =
-            found ? uint64_t(track_number) :
-                    ((entry & ~(uint64_t(0x7) << skipped_shift)) | (uint64_t(skipped + 1) << skipped_shift));
-          ring[(cnt.ttf + ((excl >> 10) & 0x3FFu)) % max_tracks_to_follow] = value;
+        else {
+          // requeued as it is, with skipped + 1
+          entry = (entry & ~(uint64_t(skipped_mask) << skipped_shift)) |
+                  (uint64_t((skipped + 1) & skipped_mask) << skipped_shift);
         }
+        if (enqueue) ring.append(cnt.ttf + ((excl >> 10) & 0x3FFu)) = entry;
         if (three) {
           const unsigned slot = cnt.n_three + ((excl >> 20) & 0x3FFu);
           if (slot < track_limit) {
@@ -770,7 +631,6 @@ namespace velo {
     return chi2 * 0.5f;
   }
 
-  // The three module pairs of a step (first, first - 1, first - 2), read by every thread.
   // The event's module pairs into shared memory, last first (threads 0-25; a barrier follows).
   __device__ __forceinline__ void module_pairs(
     ModulePair* mps, const Geometry* g, const unsigned* start, const unsigned* num, unsigned hit_offset)
@@ -786,16 +646,26 @@ namespace velo {
     }
   }
 
-  // Seeding, forwarding and the tail of one event over staged hits (hit_used clear):
+  // The bucket table of a module pair and its phi values, into its slot (a barrier follows).
+  __device__ __forceinline__ void load_pair(SearchShared& s, const Hits& h, const ModulePair& m)
+  {
+    if (m.hit_num <= phi_capacity)
+      for (unsigned i = threadIdx.x; i < m.hit_num; i += blockDim.x)
+        s.phi[m.table][i] = h.phi(m.hit_start + i);
+    build_bucket_table_of(s.bucket[m.table], [h](unsigned j) { return h.phi(j); }, m.hit_start, m.hit_num);
+  }
+
+  // Seeding, forwarding and the tail of one event over staged hits (used bits clear):
   // SearchByTriplet.cu:165-264.  Returns the event's counters; the track containers hold
-  // its tracks and three-hit tracks.
-  template<unsigned LPH, bool GATED, typename Shared>
+  // its tracks and three-hit tracks, s.track_hits the hits of the former.
+  template<bool GATED, typename Shared, typename RingT>
   __device__ __forceinline__ Counters search_pass(
     const SearchParams& p,
     Shared& s,
-    uint64_t* ring,
+    RingT& ring,
     const Constants& k,
     const Hits& h,
+    const UsedBits& used,
     const unsigned* start,
     const unsigned* num,
     unsigned hit_offset,
@@ -813,72 +683,73 @@ namespace velo {
     unsigned first = n_module_pairs - 1;
     const ModulePair* md = s.mps;
     for (unsigned i = 0; i < 2; ++i)
-      build_bucket_table_of(s.bucket[md[i].table], [h](unsigned j) { return h.phi(j); }, md[i].hit_start, md[i].hit_num);
+      load_pair(s, h, md[i]);
 
     // One step per module pair first = 25 ... 2 (the first without forwarding), with a single
     // copy of the seeding code.
-    unsigned last_ttf = 0;
+    unsigned last_ttf = 0, track_hits = 0;
     const unsigned window = GATED && gate != nullptr && p.seed_window ? p.seed_window : 4u;
     for (;;) {
-      // the table of module pair first - 2 replaces that of first + 1, last read by the
-      // previous step's seeding
-      build_bucket_table_of(s.bucket[md[2].table], [h](unsigned j) { return h.phi(j); }, md[2].hit_start, md[2].hit_num);
+      // module pair first - 2 takes the slot of first + 1, last read by the previous step's
+      // seeding before its last barrier
+      load_pair(s, h, md[2]);
       const bool forward = first < n_module_pairs - 1;
       const unsigned prev_ttf = last_ttf;
-      if (forward) last_ttf = cnt.ttf;
+      if (forward) {
+        last_ttf = cnt.ttf;
+        ring.next_generation(cnt.ttf);
+      }
       if (threadIdx.x == 0) s.local_hits = 0;
       __syncthreads(); // ring entries of the last seeding, the new bucket table
       if (forward) {
-        forwarding(s, ring, cnt, k, h, md[2], prev_ttf, last_ttf - prev_ttf, tracks, track_limit, three_hit, p.status);
+        forwarding(
+          s, ring, cnt, k, h, used, md[2], prev_ttf, last_ttf - prev_ttf, tracks, track_limit, three_hit, track_hits,
+          p.status);
         // The ring holds 2048 entries; beyond that the reference overwrites entries it has
         // not read yet, an order-dependent outcome this kernel does not reproduce.
         if (threadIdx.x == 0 && cnt.ttf - prev_ttf > max_tracks_to_follow) set_error(p.status, err_ttf_overflow);
-        __syncthreads(); // hit_used flags written by forwarding
+        __syncthreads(); // used bits set by forwarding
       }
-      if constexpr (LPH == 0) seeding_flat<GATED>(s, ring, cnt, k, h, md, forward ? window : 8u, gate, outcome);
-      else seeding<LPH>(s, ring, cnt, k, h, md, forward ? 4u : 8u);
+      seeding<GATED>(s, ring, cnt, k, h, used, md, forward ? window : 8u, gate, outcome);
       if (forward && threadIdx.x == 0 && cnt.ttf - last_ttf > max_tracks_to_follow) set_error(p.status, err_ttf_overflow);
       if (--first <= 1) break;
       ++md;
     }
+    track_hits = __reduce_add_sync(0xFFFFFFFFu, track_hits);
+    if ((threadIdx.x & 31u) == 0) atomicAdd(&s.track_hits, track_hits);
     __syncthreads(); // ring entries of the last seeding
 
     // Tail: seeds still in flight become three-hit tracks (SearchByTriplet.cu:247-264)
-    {
-      const unsigned prev_ttf = last_ttf;
-      last_ttf = cnt.ttf;
-      const unsigned diff = last_ttf - prev_ttf;
-      for (unsigned c0 = 0; c0 < diff; c0 += blockDim.x) {
-        const unsigned kk = c0 + threadIdx.x;
-        uint64_t entry = 0;
-        bool seed = false;
-        if (kk < diff) {
-          entry = ring[(prev_ttf + kk) % max_tracks_to_follow];
-          seed = (entry & seed_flag) != 0;
-        }
-        unsigned total;
-        const unsigned excl = scan_flags<1>(s, cnt, seed, false, false, total);
-        if (seed) {
-          const unsigned slot = cnt.n_three + excl;
-          if (slot < track_limit) {
-            three_hit[slot] = TrackletHits {{static_cast<uint16_t>(entry & 0xFFFFu),
-                                             static_cast<uint16_t>((entry >> 16) & 0xFFFFu),
-                                             static_cast<uint16_t>((entry >> 32) & 0xFFFFu)}};
-          }
-          else {
-            set_error(p.status, err_track_capacity);
-          }
-        }
-        cnt.n_three += total;
+    const unsigned diff = cnt.ttf - last_ttf;
+    for (unsigned c0 = 0; c0 < diff; c0 += blockDim.x) {
+      const unsigned kk = c0 + threadIdx.x;
+      uint64_t entry = 0;
+      bool seed = false;
+      if (kk < diff) {
+        entry = ring.append(last_ttf + kk);
+        seed = (entry & seed_flag) != 0;
       }
+      unsigned total;
+      const unsigned excl = scan_flags<1>(s, cnt, seed, false, false, total);
+      if (seed) {
+        const unsigned slot = cnt.n_three + excl;
+        if (slot < track_limit) {
+          three_hit[slot] = TrackletHits {{static_cast<uint16_t>(entry & 0xFFFFu),
+                                           static_cast<uint16_t>((entry >> 16) & 0xFFFFu),
+                                           static_cast<uint16_t>((entry >> 32) & 0xFFFFu)}};
+        }
+        else {
+          set_error(p.status, err_track_capacity);
+        }
+      }
+      cnt.n_three += total;
     }
-
     return cnt;
   }
 
-  template<unsigned LPH, bool SMEM, bool GATED, typename Shared>
+  template<bool SMEM, bool GATED, typename Shared, typename RingT>
   __device__ __forceinline__ void
-  search_event(const SearchParams& p, Shared& s, uint64_t* ring, unsigned char* dsmem, unsigned e)
+  search_event(const SearchParams& p, Shared& s, RingT ring, unsigned char* dsmem, unsigned e)
   {
     const unsigned n = p.n_events;
     const unsigned* start = p.offsets_estimated_input_size + e * n_module_pairs;
@@ -906,8 +777,12 @@ namespace velo {
     TrackletHits* three_hit = p.three_hit_tracks + to;
 
     // Stage the hits as 16-byte records: shared memory when they fit (SMEM), else the
-    // event's global slice (16 bytes per estimated hit).
+    // event's global slice (16 bytes per estimated hit).  All unused.
     const Hits h {SMEM ? reinterpret_cast<uint4*>(dsmem) : reinterpret_cast<uint4*>(p.hit_scratch) + hit_offset};
+    const UsedBits used {n_hits <= used_capacity ? s.used :
+                                                   reinterpret_cast<uint32_t*>(p.used_scratch + size_t(24) * hit_offset)};
+    for (unsigned i = threadIdx.x; i <= (n_hits + 31u) / 32u; i += blockDim.x)
+      used.w[i] = 0;
     {
       const ClusterView g {const_cast<char*>(p.sorted_container), T};
       // read once: streaming loads (evict first), which leave L2 to the staged hits
@@ -936,8 +811,8 @@ namespace velo {
       }
     }
     uint8_t* outcome = GATED && p.h1_outcome != nullptr ? p.h1_outcome + hit_offset : nullptr;
-    Counters cnt =
-      search_pass<LPH, GATED>(p, s, ring, k, h, start, num, hit_offset, tracks, track_limit, three_hit, gate, outcome);
+    Counters cnt = search_pass<GATED>(
+      p, s, ring, k, h, used, start, num, hit_offset, tracks, track_limit, three_hit, gate, outcome);
     if (p.seed_stats != nullptr && threadIdx.x == 0) {
       p.seed_stats[3 * e] = s.candidates;
       p.seed_stats[3 * e + 1] = s.searched;
@@ -955,7 +830,7 @@ namespace velo {
     {
       uint8_t* g_used = reinterpret_cast<uint8_t*>(p.hit_used) + hit_offset;
       for (unsigned i = threadIdx.x; i < n_hits; i += blockDim.x)
-        g_used[i] = h.flags(i) & flag_used;
+        g_used[i] = used[i];
     }
     __syncthreads();
 
@@ -969,10 +844,10 @@ namespace velo {
       TrackletHits t {};
       if (i < n_in) {
         t = three_hit[i];
-        const Hit r[3] = {h[t.hits[0]], h[t.hits[1]], h[t.hits[2]]};
-        const bool any_used = ((r[0].flags | r[1].flags | r[2].flags) & flag_used) != 0;
-        const float chi2 = means_square_fit_chi2(r);
-        keep = !any_used && chi2 < k.max_chi2;
+        if (!used[t.hits[0]] && !used[t.hits[1]] && !used[t.hits[2]]) {
+          const Hit r[3] = {h[t.hits[0]], h[t.hits[1]], h[t.hits[2]]};
+          keep = means_square_fit_chi2(r) < k.max_chi2;
+        }
       }
       unsigned total;
       const unsigned excl = scan_flags<1>(s, cnt, keep, false, false, total);
@@ -987,53 +862,49 @@ namespace velo {
     if (!SMEM) discard_l2(h.r, size_t(16) * n_hits);
   }
 
-  // One instantiation per (block size, lanes per seed, ring place); the chain launches the one
-  // its launch configuration names (autotuned).  Events whose hits fit the shared-memory
-  // capacity run the shared-memory body, the others the global-scratch body.  The ring of
-  // tracks to follow (2048 entries, 16 KiB) sits in shared memory, or with RING = 1 in this
-  // CTA's slice of a global scratch (persistent launches only: the slice is the CTA's index),
-  // which leaves room for more resident CTAs per SM.
-  // Flat-seeding kernels are register-capped for 2048 threads per SM (32 registers, some
-  // spills): with the hits and the ring staged through L2 shared memory no longer limits the
-  // CTAs per SM, and the extra resident events hide more latency than the spills cost
-  // (measured per 16000-event launch: 4.01 ms at twelve 128-thread CTAs and 40 registers,
-  // 3.83 ms at sixteen and 32 registers; the smaller the shared-memory footprint, the larger
-  // the L1 that caches the hit records).
-  template<unsigned THREADS, unsigned LPH, unsigned RING>
-  __global__ void __launch_bounds__(THREADS, LPH == 0 ? 2048 / THREADS : 1) search_by_triplet_kernel(SearchParams p)
+  // One instantiation per (block size, ring place); the chain launches the one its launch
+  // configuration names (autotuned).  Events whose hits fit the shared-memory capacity run the
+  // shared-memory body, the others the global-scratch body.  The ring of tracks to follow (2048
+  // entries, 16 KiB) sits in shared memory, or with RING = 1 in this CTA's slice of a global
+  // scratch (persistent launches only: the slice is the CTA's index) behind near_entries of each
+  // step in shared memory, which leaves room for more resident CTAs per SM.
+  // Issue-bound.  Register-capped for 2048 threads per SM (32 registers): with the hits staged
+  // through L2 shared memory does not limit the CTAs per SM, and the resident events hide more
+  // latency than the cap costs (16000 events: 2.36 ms; twelve CTAs per SM at 40 registers 2.51,
+  // eight at 64 registers 2.83).  The seeding by used bits, against used flags in the hit records,
+  // an index of the unused hits and a packed list of doublets per step (ten barriers a step
+  // instead of five): 3.01 -> 2.36 ms, 10 events 313 -> 245 us.
+  template<unsigned THREADS, unsigned RING, bool GATED>
+  __device__ __forceinline__ void search_events(const SearchParams& p)
   {
     extern __shared__ __align__(128) unsigned char dsmem[];
-    __shared__ std::conditional_t<LPH == 0, SearchSharedFlatPlain<THREADS>, SearchShared> s;
-    __shared__ uint64_t ring_smem[RING ? 1 : max_tracks_to_follow];
-    uint64_t* ring = RING ? p.ring_scratch + size_t(blockIdx.x) * max_tracks_to_follow : ring_smem;
+    __shared__ std::conditional_t<GATED, SearchSharedGated, SearchShared> s;
+    __shared__ uint64_t near_ring[RING ? 2 * near_entries : max_tracks_to_follow];
+    const Ring<RING != 0> ring {RING ? p.ring_scratch + size_t(blockIdx.x) * max_tracks_to_follow : near_ring, near_ring, 0, 0};
     for_each_event(p.queue, p.n_events, [&](unsigned e, unsigned) {
       const unsigned* start = p.offsets_estimated_input_size + e * n_module_pairs;
       const unsigned n_hits = start[n_module_pairs] - start[0];
-      if (n_hits <= p.smem_hit_capacity) search_event<LPH, true, false>(p, s, ring, dsmem, e);
-      else search_event<LPH, false, false>(p, s, ring, dsmem, e);
+      if (n_hits <= p.smem_hit_capacity) search_event<true, GATED>(p, s, ring, dsmem, e);
+      else search_event<false, GATED>(p, s, ring, dsmem, e);
     });
   }
 
-  // The learned search: flat seeding behind the seed gate (with seed_gate null, the plain
+  template<unsigned THREADS, unsigned RING>
+  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) search_by_triplet_kernel(SearchParams p)
+  {
+    search_events<THREADS, RING, false>(p);
+  }
+
+  // The learned search: the seeding behind the seed gate (with seed_gate null, the plain
   // search, recording each seed candidate's outcome when h1_outcome is set).  The gate costs
   // one byte read per candidate, so this kernel keeps the plain kernel's register budget.
   template<unsigned THREADS, unsigned RING>
   __global__ void __launch_bounds__(THREADS, 2048 / THREADS) search_by_triplet_gated_kernel(SearchParams p)
   {
-    extern __shared__ __align__(128) unsigned char dsmem[];
-    __shared__ SearchSharedFlatPlain<THREADS, true> s;
-    __shared__ uint64_t ring_smem[RING ? 1 : max_tracks_to_follow];
-    uint64_t* ring = RING ? p.ring_scratch + size_t(blockIdx.x) * max_tracks_to_follow : ring_smem;
-    for_each_event(p.queue, p.n_events, [&](unsigned e, unsigned) {
-      const unsigned* start = p.offsets_estimated_input_size + e * n_module_pairs;
-      const unsigned n_hits = start[n_module_pairs] - start[0];
-      if (n_hits <= p.smem_hit_capacity) search_event<0, true, true>(p, s, ring, dsmem, e);
-      else search_event<0, false, true>(p, s, ring, dsmem, e);
-    });
+    search_events<THREADS, RING, true>(p);
   }
 
-#define VELO_SEARCH_CONFIG(T, L, R)                                              \
-  template __global__ void search_by_triplet_kernel<T, L, R>(SearchParams p);
+#define VELO_SEARCH_CONFIG(T, R) template __global__ void search_by_triplet_kernel<T, R>(SearchParams p);
   VELO_SEARCH_CONFIGS(VELO_SEARCH_CONFIG)
 #undef VELO_SEARCH_CONFIG
 #define VELO_GATED_CONFIG(T, R) template __global__ void search_by_triplet_gated_kernel<T, R>(SearchParams p);
