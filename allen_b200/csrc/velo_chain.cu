@@ -208,7 +208,7 @@ struct SearchVariant {
   SearchKernel fn;
 };
 static const SearchVariant search_variants[] = {
-#define VELO_SEARCH_VARIANT(T, R) {T, R, velo::search_by_triplet_kernel<T, R>},
+#define VELO_SEARCH_VARIANT(T, R) {T, R, velo::search_by_triplet_kernel<T, R, 2048>},
   VELO_SEARCH_CONFIGS(VELO_SEARCH_VARIANT)
 #undef VELO_SEARCH_VARIANT
 };
@@ -235,8 +235,8 @@ static constexpr size_t n_sensors_total = velo::n_sensors;
 static SearchKernel gated_search_kernel(unsigned threads, unsigned ring_global)
 {
 #define VELO_GATED_VARIANT(T, R) \
-  if (threads == T && ring_global == R) return velo::search_by_triplet_gated_kernel<T, R>;
-  VELO_GATED_CONFIGS(VELO_GATED_VARIANT)
+  if (threads == T && ring_global == R) return velo::search_by_triplet_gated_kernel<T, R, 2048>;
+  VELO_SEARCH_CONFIGS(VELO_GATED_VARIANT)
 #undef VELO_GATED_VARIANT
   return nullptr;
 }
@@ -282,7 +282,10 @@ struct VeloChain {
   unsigned seed_window = 0;                                   // learned mode: h0 candidates per seed candidate
   unsigned resident_kalman = 0;                               // Kalman CTAs resident on the device
   unsigned resident_export = 0;                               // half-layout export CTAs
+  unsigned sms = 0;
   unsigned resident_estimate = 0, resident_cluster = 0, resident_search = 0; // CTAs that fit the device
+  // the same of the kernels for slices of few events (persistent launches), 0: not for this configuration
+  unsigned resident_few_estimate = 0, resident_few_cluster = 0, resident_few_search = 0;
 
   // workspace
   DeviceBuffer<unsigned long long> bank_index_key;
@@ -531,6 +534,8 @@ namespace {
       return persistent ? WorkQueue {c->queue_next.p + k, c->event_order.p, c->events_per_claim} : WorkQueue {};
     };
     auto grid = [&](unsigned resident) { return persistent ? std::min(n, std::max(resident, 1u)) : n; };
+    // the kernels with more registers for slices of few events (velo_kernels.cuh)
+    const bool few = persistent && n <= few_events_per_sm * c->sms;
     if (persistent) {
       VELO_CUDA(cudaMemsetAsync(c->queue_next.p, 0, 3 * sizeof(unsigned), stream));
     }
@@ -590,7 +595,8 @@ namespace {
       ep.lists = c->lists.p;
       ep.queue = queue(0);
       VELO_CUDA(cudaMemsetAsync(c->list_alloc.p, 0, sizeof(unsigned), stream));
-      estimate_kernel<<<grid(c->resident_estimate), decode_threads, 0, stream>>>(ep);
+      if (few) estimate_kernel<few_decode_threads><<<grid(c->resident_few_estimate), decode_threads, 0, stream>>>(ep);
+      else estimate_kernel<2048><<<grid(c->resident_estimate), decode_threads, 0, stream>>>(ep);
       VELO_CUDA(cudaGetLastError());
       VELO_CUDA(mark());
 
@@ -620,9 +626,11 @@ namespace {
       const unsigned cluster_smem = cluster_sort_smem(std::max(c->cluster_stage_capacity, min_cluster_stage));
       cp.queue = queue(1);
       if (c->cluster_threads == 128)
-        cluster_sort_kernel<128><<<grid(c->resident_cluster), 128, cluster_smem, stream>>>(cp);
+        cluster_sort_kernel<128, 2048><<<grid(c->resident_cluster), 128, cluster_smem, stream>>>(cp);
+      else if (few)
+        cluster_sort_kernel<256, few_decode_threads><<<grid(c->resident_few_cluster), 256, cluster_smem, stream>>>(cp);
       else
-        cluster_sort_kernel<256><<<grid(c->resident_cluster), 256, cluster_smem, stream>>>(cp);
+        cluster_sort_kernel<256, 2048><<<grid(c->resident_cluster), 256, cluster_smem, stream>>>(cp);
       VELO_CUDA(cudaGetLastError());
       VELO_CUDA(mark());
     }
@@ -688,8 +696,14 @@ namespace {
       const SearchVariant* v = find_search_variant(c->search_threads, c->search_lanes, c->search_ring_global);
       if (!fn && !v) return fail(VELO_ERR_ARGUMENT, "no compiled search kernel for this launch configuration");
       void* args[] = {&sp};
-      VELO_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(fn ? fn : v->fn), dim3(grid(c->resident_search)),
-                                 dim3(c->search_threads), args, search_smem, stream));
+      SearchKernel kernel = fn ? fn : v->fn;
+      unsigned resident = c->resident_search;
+      if (few && c->resident_few_search) {
+        kernel = fn ? search_by_triplet_gated_kernel<128, 1, few_events_threads> : search_by_triplet_kernel<128, 1, few_events_threads>;
+        resident = c->resident_few_search;
+      }
+      VELO_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(kernel), dim3(grid(resident)), dim3(c->search_threads), args,
+                                 search_smem, stream));
     }
     if (c->records) {
       // training records: the features of the candidates the search met, with its outcomes
@@ -773,27 +787,38 @@ namespace {
     using namespace velo;
     const int cluster_smem = int(cluster_sort_smem(std::max(c->cluster_stage_capacity, min_cluster_stage)));
     const int search_smem = int(c->search_hit_capacity * search_hit_bytes);
-    VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(cluster_sort_kernel<128>), cluster_smem));
-    VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(cluster_sort_kernel<256>), cluster_smem));
+    const auto cluster_128 = cluster_sort_kernel<128, 2048>, cluster_256 = cluster_sort_kernel<256, 2048>,
+               cluster_few = cluster_sort_kernel<256, few_decode_threads>;
+    for (auto k : {cluster_128, cluster_256, cluster_few})
+      VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(k), cluster_smem));
+    const SearchKernel few_plain = search_by_triplet_kernel<128, 1, few_events_threads>,
+                       few_gated = search_by_triplet_gated_kernel<128, 1, few_events_threads>;
+    for (SearchKernel k : {few_plain, few_gated})
+      VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(k), search_smem));
     for (const auto& v : search_variants)
       VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(v.fn), search_smem));
 #define VELO_GATED_LIMIT(T, R) \
-    VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(search_by_triplet_gated_kernel<T, R>), search_smem));
-    VELO_GATED_CONFIGS(VELO_GATED_LIMIT)
+    VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(search_by_triplet_gated_kernel<T, R, 2048>), search_smem));
+    VELO_SEARCH_CONFIGS(VELO_GATED_LIMIT)
 #undef VELO_GATED_LIMIT
     // CTAs of each kernel resident on the device at once: the grid of a persistent launch
     int sms = 0, per_sm = 0;
     VELO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, estimate_kernel, decode_threads, 0));
+    c->sms = unsigned(sms);
+    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, estimate_kernel<2048>, decode_threads, 0));
     c->resident_estimate = unsigned(std::max(per_sm, 1) * sms);
+    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, estimate_kernel<few_decode_threads>, decode_threads, 0));
+    c->resident_few_estimate = unsigned(std::max(per_sm, 1) * sms);
+    VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_few, 256, cluster_smem));
+    c->resident_few_cluster = unsigned(std::max(per_sm, 1) * sms);
     VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kalman_filter_kernel, kalman_threads, 0));
     c->resident_kalman = unsigned(std::max(per_sm, 1) * sms);
     VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, export_half_kernel, 256, 0));
     c->resident_export = unsigned(std::max(per_sm, 1) * sms);
     if (c->cluster_threads == 128)
-      VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_sort_kernel<128>, 128, cluster_smem));
+      VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_128, 128, cluster_smem));
     else
-      VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_sort_kernel<256>, 256, cluster_smem));
+      VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cluster_256, 256, cluster_smem));
     c->resident_cluster = unsigned(std::max(per_sm, 1) * sms);
     const SearchVariant* v = find_search_variant(c->search_threads, c->search_lanes, c->search_ring_global);
     const SearchKernel learned = gated_search_kernel(c->search_threads, c->search_ring_global);
@@ -802,11 +827,17 @@ namespace {
       VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, int(c->search_threads), search_smem));
       c->resident_search = unsigned(std::max(per_sm, 1) * sms);
     }
+    c->resident_few_search = 0;
+    if (c->search_threads == 128 && c->search_ring_global) {
+      VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, c->learned || c->records ? few_gated : few_plain, 128, search_smem));
+      c->resident_few_search = unsigned(std::max(per_sm, 1) * sms);
+    }
     // the global rings: one per CTA of the persistent search grid (plain or learned kernel,
     // whichever has more resident CTAs, so that switching modes needs no new allocation)
     if (c->search_ring_global) {
       size_t ctas = 0;
-      for (SearchKernel k : {v ? v->fn : nullptr, learned}) {
+      for (SearchKernel k : {v ? v->fn : nullptr, learned, few_plain, few_gated}) {
         if (!k) continue;
         VELO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(c->search_threads), search_smem));
         ctas = std::max(ctas, size_t(std::max(per_sm, 1)) * sms);

@@ -693,10 +693,13 @@ namespace velo {
   // Issue-bound (80 % of the issue slots).  16000 events of 2540 SPs: 1.06 ms (reading and parsing
   // 0.14, pass 1 0.24, pass 2 0.37, pass 3 0.31), where this kernel without pass 3 took 0.79 and the
   // clustering kernel twice as long as now.
-  __global__ void __launch_bounds__(decode_threads, 2048 / decode_threads) estimate_kernel(EstimateParams p)
+  template<unsigned SM_THREADS>
+  __global__ void __launch_bounds__(decode_threads, SM_THREADS / decode_threads) estimate_kernel(EstimateParams p)
   {
     for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { estimate_event(p, e); });
   }
+  template __global__ void estimate_kernel<2048>(EstimateParams p);
+  template __global__ void estimate_kernel<few_decode_threads>(EstimateParams p);
 
   // ------------------------------------------------------------------------------------
   // cluster_sort_kernel
@@ -958,14 +961,15 @@ namespace velo {
   // the clusters written out in the order they were staged, 1.31 ms.  Written out from a staging
   // without any order (a scattered store per value) the sort alone took 0.91 ms.
   // Capped for 2048 threads per SM (32 registers; 40 or 48 registers: 0.69, 0.71 ms).
-  template<unsigned THREADS>
-  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) cluster_sort_kernel(const __grid_constant__ ClusterSortParams p)
+  template<unsigned THREADS, unsigned SM_THREADS>
+  __global__ void __launch_bounds__(THREADS, SM_THREADS / THREADS) cluster_sort_kernel(const __grid_constant__ ClusterSortParams p)
   {
     static_assert(THREADS == 128 || THREADS == 256, "block size");
     for_each_event(p.queue, p.in.n_events, [&](unsigned e, unsigned) { cluster_sort_event<THREADS>(p, e); });
   }
-  template __global__ void cluster_sort_kernel<128>(const __grid_constant__ ClusterSortParams p);
-  template __global__ void cluster_sort_kernel<256>(const __grid_constant__ ClusterSortParams p);
+  template __global__ void cluster_sort_kernel<128, 2048>(const __grid_constant__ ClusterSortParams p);
+  template __global__ void cluster_sort_kernel<256, 2048>(const __grid_constant__ ClusterSortParams p);
+  template __global__ void cluster_sort_kernel<256, few_decode_threads>(const __grid_constant__ ClusterSortParams p);
 
   // Before the estimate kernel.  Block 0: the events of the slice by raw size, largest first (a
   // counting sort over 1024 size classes of 64 bytes; order within a class is arbitrary), when

@@ -168,16 +168,23 @@ namespace velo {
     return cluster_sort_counter_offset(cap) + ((sort_counters * 2 + 15u) & ~15u);
   }
 
+  // SM_THREADS: the threads per SM a kernel's registers are capped for.  2048 (32 registers) for
+  // slices of many events, where the resident events hide the latency of one another; fewer
+  // (few_events_threads, few_decode_threads: no spills, more loads in flight) for slices of no more
+  // events than few_events_per_sm per SM, which leave an SM to its events' latency anyway.  1000
+  // events: estimate 166 -> 137 us, clustering 82 -> 70, search 437 -> 384; above that line the
+  // second wave costs more (2000 events of 8200 SPs: search 1.74 ms, with 64 registers 1.87).
+  constexpr unsigned few_events_threads = 1024, few_decode_threads = 1280, few_events_per_sm = 8;
+  template<unsigned SM_THREADS>
   __global__ void estimate_kernel(EstimateParams p);
-  template<unsigned THREADS> // 128 or 256
+  template<unsigned THREADS, unsigned SM_THREADS> // 128 or 256
   __global__ void cluster_sort_kernel(const __grid_constant__ ClusterSortParams p);
   // RING = 1: the ring of tracks to follow in global scratch (persistent launches)
-  template<unsigned THREADS, unsigned RING>
+  template<unsigned THREADS, unsigned RING, unsigned SM_THREADS>
   __global__ void search_by_triplet_kernel(SearchParams p);
   // the seeding behind the learned seed gate (and seed-candidate outcome recording)
-  template<unsigned THREADS, unsigned RING>
+  template<unsigned THREADS, unsigned RING, unsigned SM_THREADS>
   __global__ void search_by_triplet_gated_kernel(SearchParams p);
-#define VELO_GATED_CONFIGS(X) X(128, 0) X(256, 0) X(512, 0) X(128, 1) X(256, 1) X(96, 1) X(64, 1)
 #define VELO_SEARCH_CONFIGS(X) X(128, 0) X(256, 0) X(512, 0) X(128, 1) X(256, 1) X(96, 1) X(64, 1)
   __global__ void consolidate_kernel(ConsolidateParams p);
   // ---- retina-cluster decoding (VPRetinaCluster banks) ----

@@ -89,7 +89,7 @@ namespace {
       const cudaError_t e = cudaGetSymbolAddress(&ptr, velo_noalloc_scratch);
       if (e != cudaSuccess) return fail(VELO_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
       const int cluster_smem = int(velo::cluster_sort_smem(cluster_stage_capacity));
-      if (velo::raise_dynamic_smem_limit(reinterpret_cast<const void*>(velo::cluster_sort_kernel<velo::decode_threads>), cluster_smem) !=
+      if (velo::raise_dynamic_smem_limit(reinterpret_cast<const void*>(velo::cluster_sort_kernel<velo::decode_threads, 2048>), cluster_smem) !=
             cudaSuccess)
         return fail(VELO_ERR_CUDA, "cannot set the kernels' shared-memory limits");
       scratch_address[device] = static_cast<unsigned char*>(ptr);
@@ -187,7 +187,7 @@ VeloStatus velo_decode_noalloc(
   ep.list_alloc = reinterpret_cast<unsigned*>(scratch + off_list_alloc);
   ep.lists = reinterpret_cast<uint4*>(scratch + off_lists);
   event_order_kernel<<<event_order_grid(n, true), scan_threads, 0, stream>>>(in, nullptr, bank_index_stride(n), bank_index);
-  estimate_kernel<<<n, decode_threads, 0, stream>>>(ep);
+  estimate_kernel<2048><<<n, decode_threads, 0, stream>>>(ep);
 
   ScanParams sp {};
   sp.jobs[0] = {event_estimate, event_base, n};
@@ -214,7 +214,7 @@ VeloStatus velo_decode_noalloc(
   cp.smem_cluster_capacity = cluster_stage_capacity;
   cp.cluster_capacity = static_cast<unsigned>(bound);
   const unsigned cluster_smem = cluster_sort_smem(cluster_stage_capacity);
-  cluster_sort_kernel<decode_threads><<<n, decode_threads, cluster_smem, stream>>>(cp);
+  cluster_sort_kernel<decode_threads, 2048><<<n, decode_threads, cluster_smem, stream>>>(cp);
   const cudaError_t launch = cudaGetLastError();
   if (launch != cudaSuccess) return fail(VELO_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(launch));
   if (dev_status && cudaMemcpyAsync(dev_status, status, sizeof(unsigned), cudaMemcpyDeviceToDevice, stream) != cudaSuccess)

@@ -871,7 +871,8 @@ namespace velo {
   // Issue-bound.  Register-capped for 2048 threads per SM (32 registers): with the hits staged
   // through L2 shared memory does not limit the CTAs per SM, and the resident events hide more
   // latency than the cap costs (16000 events: 2.36 ms; twelve CTAs per SM at 40 registers 2.51,
-  // eight at 64 registers 2.83).  The seeding by used bits, against used flags in the hit records,
+  // eight at 64 registers 2.83).  Slices that eight CTAs per SM hold take 64 registers (128
+  // threads with global rings: 1000 events 437 -> 384 us, 10 events 245 -> 235 us).  The seeding by used bits, against used flags in the hit records,
   // an index of the unused hits and a packed list of doublets per step (ten barriers a step
   // instead of five): 3.01 -> 2.36 ms, 10 events 313 -> 245 us.
   template<unsigned THREADS, unsigned RING, bool GATED>
@@ -889,8 +890,8 @@ namespace velo {
     });
   }
 
-  template<unsigned THREADS, unsigned RING>
-  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) search_by_triplet_kernel(SearchParams p)
+  template<unsigned THREADS, unsigned RING, unsigned SM_THREADS>
+  __global__ void __launch_bounds__(THREADS, SM_THREADS / THREADS) search_by_triplet_kernel(SearchParams p)
   {
     search_events<THREADS, RING, false>(p);
   }
@@ -898,17 +899,18 @@ namespace velo {
   // The learned search: the seeding behind the seed gate (with seed_gate null, the plain
   // search, recording each seed candidate's outcome when h1_outcome is set).  The gate costs
   // one byte read per candidate, so this kernel keeps the plain kernel's register budget.
-  template<unsigned THREADS, unsigned RING>
-  __global__ void __launch_bounds__(THREADS, 2048 / THREADS) search_by_triplet_gated_kernel(SearchParams p)
+  template<unsigned THREADS, unsigned RING, unsigned SM_THREADS>
+  __global__ void __launch_bounds__(THREADS, SM_THREADS / THREADS) search_by_triplet_gated_kernel(SearchParams p)
   {
     search_events<THREADS, RING, true>(p);
   }
 
-#define VELO_SEARCH_CONFIG(T, R) template __global__ void search_by_triplet_kernel<T, R>(SearchParams p);
+#define VELO_SEARCH_CONFIG(T, R)                                                  \
+  template __global__ void search_by_triplet_kernel<T, R, 2048>(SearchParams p);  \
+  template __global__ void search_by_triplet_gated_kernel<T, R, 2048>(SearchParams p);
   VELO_SEARCH_CONFIGS(VELO_SEARCH_CONFIG)
 #undef VELO_SEARCH_CONFIG
-#define VELO_GATED_CONFIG(T, R) template __global__ void search_by_triplet_gated_kernel<T, R>(SearchParams p);
-  VELO_GATED_CONFIGS(VELO_GATED_CONFIG)
-#undef VELO_GATED_CONFIG
+  template __global__ void search_by_triplet_kernel<128, 1, few_events_threads>(SearchParams p);
+  template __global__ void search_by_triplet_gated_kernel<128, 1, few_events_threads>(SearchParams p);
 
 } // namespace velo
