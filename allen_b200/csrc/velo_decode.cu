@@ -240,21 +240,36 @@ namespace velo {
   // compares every pair of a bank's SPs: estimate and clustering together 2.79 -> 2.10 ms for
   // 16000 events of 2540 SPs, 1.75 -> 1.06 ms for 2000 of 8200 SPs, version 4, 78 SPs per bank.)
   // ------------------------------------------------------------------------------------
-  // visit(w) for the SPs among bank_words[0, n) with lo <= ((w >> 8) & key_mask) <= lo + span, in order.
-  template<typename Visit>
-  __device__ __forceinline__ void
-  scan_keys(const uint32_t* bank_words, unsigned n, uint32_t lo, uint32_t span, uint32_t key_mask, Visit&& visit)
+  // visit(w) for the SPs among words[0, n) but words[self] with lo <= ((w >> 8) & key_mask) <= lo + span,
+  // in order (self >= n: none left out).  Eight keys at a time: up to seven words behind the last
+  // are read, and not used, when PAD says that they may be.
+  template<bool PAD, typename Visit>
+  __device__ __forceinline__ void scan_keys(
+    const uint32_t* words, unsigned n, unsigned self, uint32_t lo, uint32_t span, uint32_t key_mask, Visit&& visit)
   {
     const uint32_t mask = key_mask << 8;
     lo <<= 8;
     span <<= 8;
     for (unsigned base = 0; base < n; base += 32) {
-      const uint32_t* w = bank_words + base;
+      const uint32_t* w = words + base;
       const unsigned count = min(n - base, 32u);
       uint32_t inside = 0;
+      if constexpr (PAD) {
+        for (unsigned j = 0; j < count; j += 8) {
+          uint32_t eight = 0;
+#pragma unroll
+          for (unsigned q = 0; q < 8; ++q)
+            if ((w[j + q] & mask) - lo <= span) eight |= 1u << q;
+          inside |= eight << j;
+        }
+        inside &= 0xFFFFFFFFu >> (32u - count);
+      }
+      else {
 #pragma unroll 4
-      for (unsigned j = 0; j < count; ++j)
-        inside |= ((w[j] & mask) - lo <= span ? 1u : 0u) << j;
+        for (unsigned j = 0; j < count; ++j)
+          inside |= ((w[j] & mask) - lo <= span ? 1u : 0u) << j;
+      }
+      if (self - base < 32u) inside &= ~(1u << (self - base));
       for (; inside; inside &= inside - 1)
         visit(w[__ffs(inside) - 1]);
     }
@@ -267,7 +282,8 @@ namespace velo {
   // Returns up to two candidate pixel codes: bit 8 set = present, bits 0..2 = pixel.
   // ------------------------------------------------------------------------------------
   // Neighbours of either sensor of a version 4 bank count (the reference compares bits 22:8 only).
-  __device__ __forceinline__ uint32_t sp_candidates(uint32_t sp_word, const uint32_t* bank_words, unsigned n_sp)
+  template<bool PAD>
+  __device__ __forceinline__ uint32_t sp_candidates(uint32_t sp_word, const uint32_t* bank_words, unsigned n_sp, unsigned self)
   {
     const uint32_t sp_addr = (sp_word & 0x007FFF00u) >> 8;
     const uint32_t sp = sp_word & 0xFFu;
@@ -275,7 +291,7 @@ namespace velo {
     const uint32_t row = sp_addr & 0x3Fu;
     // Addresses from one row below in the same column to one row above in the next (the SP itself
     // adds nothing); a row beyond the column's ends is another column's.
-    scan_keys(bank_words, n_sp, sp_addr - 1, 66, 0x7FFFu, [&](uint32_t ow) {
+    scan_keys<PAD>(bank_words, n_sp, self, sp_addr - 1, 66, 0x7FFFu, [&](uint32_t ow) {
       const uint32_t ahead = ((ow & 0x007FFF00u) >> 8) - sp_addr;
       const bool above = row < 63 && (ahead == 1 || ahead == 65), below = row > 0 && (ahead == ~0u || ahead == 63);
       const bool next = ahead > 62 && ahead <= 65;
@@ -375,6 +391,7 @@ namespace velo {
     uint32_t x, y, n;
     bool bad;
   };
+  template<bool PAD>
   __device__ __forceinline__ ClusterSums grow_cluster(
     uint32_t sp_word, uint32_t start_loc, uint32_t sensor_number, const uint32_t* bank_words, unsigned n_sp, int version)
   {
@@ -393,7 +410,7 @@ namespace velo {
     const uint32_t key_mask = version > 3 ? 0xFFFFu : 0x7FFFu;
     const uint32_t sensor_key = version > 3 ? (sensor_number & 0x1u) << 15 : 0u;
     const uint32_t lowest = sensor_key + static_cast<uint32_t>(c_lo * 64 + r_lo);
-    scan_keys(bank_words, n_sp, lowest, 4 * 64 + 3, key_mask, [&](uint32_t ow) {
+    scan_keys<PAD>(bank_words, n_sp, 0xFFFFFFFFu, lowest, 4 * 64 + 3, key_mask, [&](uint32_t ow) {
       if ((((ow >> 8) & key_mask) ^ sensor_key) & 0x8000u) return;
       if (ow & 0x80000000u) return;
       const uint32_t oaddr = (ow & 0x007FFF00u) >> 8;
@@ -525,7 +542,7 @@ namespace velo {
     __shared__ unsigned list_at, no_list;
     // the event's SPs in bank order, when they fit: the words, with the bank as its distance
     // from the hint (127: too far) in bits 24 to 30, which SPs do not use
-    __shared__ uint32_t held[estimate_words];
+    __shared__ uint32_t held[estimate_words + 8]; // (8: scans read on)
 
     const unsigned ev = e + p.in.event_start;
     const int version = p.in.bank_version;
@@ -578,33 +595,42 @@ namespace velo {
       return words[bt.words_off[b] + f - bt.flat[b]];
     };
     for (unsigned chunk_base = 0, parity = 0; chunk_base < total_sp; chunk_base += estimate_queue, parity ^= 1u) {
-      for (unsigned f = chunk_base + threadIdx.x; f < min(chunk_base + estimate_queue, total_sp); f += blockDim.x) {
-        unsigned b;
-        const uint32_t word = sp_word(f, b);
-        unsigned clusters = 0;
-        if (word & 0x80000000u) {
-          const unsigned source_id = bt.source_id[b];
-          const unsigned mp = bank_module_pair(source_id, version);
-          if (mp < n_module_pairs) {
-            clusters = isolated_two_clusters(word & 0xFFu) ? 2u : 1u;
-            add_to_counter(est_mp, mp, clusters);
-            if (list != nullptr) {
-              // the sensor field of a version 2 or 3 channel id takes bit 9 of the source ID too, which
-              // an item has no room for
-              if (v23 && (source_id & 0x200u)) no_list = 1;
-              unsigned second;
-              const unsigned first = append_items(&isolated_count, clusters, second);
-              if (first < room) list[first] = isolated_item(word, source_id, v23, 0);
-              if (clusters > 1 && second < room) list[second] = isolated_item(word, source_id, v23, 1);
-            }
-          }
-          else {
-            set_error(p.status, err_input_capacity);
-          }
+      // (whole warps: f of lane 0 is a multiple of 32)
+      for (unsigned f = chunk_base + threadIdx.x; (f & ~31u) < min(chunk_base + estimate_queue, total_sp); f += blockDim.x) {
+        const unsigned lane = threadIdx.x & 31u;
+        unsigned b = 0, clusters = 0, mp = 0, source_id = 0;
+        uint32_t word = 0;
+        bool other = false;
+        if (f < total_sp) {
+          word = sp_word(f, b);
+          source_id = bt.source_id[b];
+          mp = bank_module_pair(source_id, version);
+          other = !(word & 0x80000000u);
+          if (mp >= n_module_pairs) set_error(p.status, err_input_capacity);
+          else if (!other) clusters = isolated_two_clusters(word & 0xFFu) ? 2u : 1u;
         }
-        else {
-          unsigned unused;
-          queue[append_items(&queue_count[parity], 1, unused)] = static_cast<uint16_t>(f - chunk_base);
+        const unsigned one = __ballot_sync(0xFFFFFFFFu, clusters > 0), two = __ballot_sync(0xFFFFFFFFu, clusters > 1);
+        const unsigned rest = __ballot_sync(0xFFFFFFFFu, other);
+        // lanes 0 to 2 add to the three counters at once: the items, the queue, and the estimate of the
+        // module pair when all isolated SPs of the warp lie in one
+        const unsigned mp0 = __shfl_sync(0xFFFFFFFFu, mp, __ffs(one) - 1);
+        const bool same = __all_sync(0xFFFFFFFFu, clusters == 0 || mp == mp0);
+        const unsigned n_items = __popc(one) + __popc(two);
+        unsigned* counter = lane == 0 ? &isolated_count : (lane == 1 ? &queue_count[parity] : est_mp + mp0);
+        const unsigned n = lane == 1 ? __popc(rest) : n_items;
+        unsigned at = 0;
+        if (lane < (same && n_items ? 3u : 2u)) at = atomicAdd(counter, n);
+        if (!same && clusters) atomicAdd(est_mp + mp, clusters);
+        const unsigned first = __shfl_sync(0xFFFFFFFFu, at, 0), first_queued = __shfl_sync(0xFFFFFFFFu, at, 1);
+        const unsigned below = (1u << lane) - 1u;
+        if (other) queue[first_queued + __popc(rest & below)] = static_cast<uint16_t>(f - chunk_base);
+        if (clusters && list != nullptr) {
+          // the sensor field of a version 2 or 3 channel id takes bit 9 of the source ID too, which
+          // an item has no room for
+          if (v23 && (source_id & 0x200u)) no_list = 1;
+          const unsigned k = first + __popc(one & below), k2 = first + __popc(one) + __popc(two & below);
+          if (k < room) list[k] = isolated_item(word, source_id, v23, 0);
+          if (clusters > 1 && k2 < room) list[k2] = isolated_item(word, source_id, v23, 1);
         }
       }
       __syncthreads();
@@ -615,8 +641,9 @@ namespace velo {
         unsigned b;
         const uint32_t word = sp_word(f, b);
         const unsigned at = bt.flat[b], source_id = bt.source_id[b];
-        const uint32_t* bank_words = in_smem ? held + at : words + bt.words_off[b];
-        const uint32_t c = sp_candidates(word, bank_words, bt.flat[b + 1] - at);
+        const unsigned n_sp = bt.flat[b + 1] - at;
+        const uint32_t c = in_smem ? sp_candidates<true>(word, held + at, n_sp, f - at) :
+                                     sp_candidates<false>(word, words + bt.words_off[b], n_sp, f - at);
         const unsigned add = ((c >> 8) & 1u) + ((c >> 24) & 1u);
         const unsigned mp = bank_module_pair(source_id, version);
         unsigned second;
@@ -642,13 +669,10 @@ namespace velo {
         // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
         const uint32_t sensor = v23 ? (source_id & 0x1FFu) : (((source_id & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
         const unsigned b2 = static_cast<unsigned>(p.bank_index_key[sensor] & 0xFFFFFFFFull);
-        const uint32_t* bank_words;
-        unsigned n_sp;
-        uint32_t start_word = word;
-        if (b2 == b) {
+        ClusterSums c;
+        if (b2 == b && in_smem) {
           const unsigned at = bt.flat[b];
-          bank_words = in_smem ? held + at : words + bt.words_off[b];
-          n_sp = bt.flat[b + 1] - at;
+          c = grow_cluster<true>(word, candidates[q] >> 10, sensor, held + at, bt.flat[b + 1] - at, version);
         }
         else {
           const unsigned index = f - bt.flat[b];
@@ -659,11 +683,9 @@ namespace velo {
             set_error(p.status, err_input_capacity);
             continue;
           }
-          bank_words = words + bank.first;
-          n_sp = bank.n_sp;
-          start_word = bank_words[index];
+          const uint32_t* bank_words = words + bank.first;
+          c = grow_cluster<false>(bank_words[index], candidates[q] >> 10, sensor, bank_words, bank.n_sp, version);
         }
-        const ClusterSums c = grow_cluster(start_word, candidates[q] >> 10, sensor, bank_words, n_sp, version);
         if (c.bad) set_error(p.status, err_bad_super_pixel);
         if (c.n > 0) {
           unsigned unused;
@@ -690,9 +712,10 @@ namespace velo {
     }
   }
 
-  // Issue-bound (80 % of the issue slots).  16000 events of 2540 SPs: 1.06 ms (reading and parsing
-  // 0.14, pass 1 0.24, pass 2 0.37, pass 3 0.31), where this kernel without pass 3 took 0.79 and the
-  // clustering kernel twice as long as now.
+  // Issue-bound (80 % of the issue slots).  16000 events of 2540 SPs: 0.97 ms.  With scans of one key
+  // at a time through a pointer to either memory, and the warp's places in list, queue and estimate
+  // claimed one after the other, 1.06 (reading and parsing 0.14, pass 1 0.24, pass 2 0.37, pass 3
+  // 0.31); without pass 3, when the clustering kernel took twice as long as now, 0.79.
   template<unsigned SM_THREADS>
   __global__ void __launch_bounds__(decode_threads, SM_THREADS / decode_threads) estimate_kernel(EstimateParams p)
   {
@@ -793,7 +816,7 @@ namespace velo {
             m.isolated(word, bank.source_id, which);
           continue;
         }
-        const uint32_t c = sp_candidates(word, w, bank.n_sp);
+        const uint32_t c = sp_candidates<false>(word, w, bank.n_sp, i);
         const uint32_t sensor =
           v23 ? (bank.source_id & 0x1FFu) : (((bank.source_id & 0x1FFu) << 1) | ((word >> 23) & 0x1u));
         // MaskedVeloClustering.cu:567-572: the candidate's bank is looked up by sensor
@@ -809,7 +832,7 @@ namespace velo {
             continue;
           }
           const uint32_t* w2 = ew.w + at.first;
-          const ClusterSums sums = grow_cluster(w2[i], code & 0x7u, sensor, w2, at.n_sp, version);
+          const ClusterSums sums = grow_cluster<false>(w2[i], code & 0x7u, sensor, w2, at.n_sp, version);
           if (sums.bad) set_error(p.status, err_bad_super_pixel);
           if (sums.n > 0) m.grown(sums.x, sums.y, sums.n, sensor);
         }
