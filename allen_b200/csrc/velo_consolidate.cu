@@ -90,13 +90,34 @@ namespace velo {
       }
       __syncthreads();
       const unsigned pos0 = hit_base + carry;
-      for (unsigned k = threadIdx.x; k < block_total; k += blockDim.x) {
-        const unsigned hi = hit_offset + chunk_hits[k];
-        if (pos0 + k >= p.track_hit_capacity || hi >= T) continue; // flagged: a track that did not fit
-        out.x(pos0 + k) = in.x(hi);
-        out.y(pos0 + k) = in.y(hi);
-        out.z(pos0 + k) = in.z(hi);
-        out.id(pos0 + k) = in.id(hi);
+      // four hits per thread in flight: the gathers' latency, not their bandwidth, is what a
+      // thread that takes one hit after the other waits for (16000 events: 0.31 -> 0.28 ms, 2000
+      // events of 380 tracks 0.14 -> 0.10)
+      constexpr unsigned flight = 4;
+      for (unsigned k0 = threadIdx.x; k0 < block_total; k0 += flight * blockDim.x) {
+        unsigned id[flight];
+        float x[flight], y[flight], z[flight];
+        bool fits[flight];
+#pragma unroll
+        for (unsigned q = 0; q < flight; ++q) {
+          const unsigned k = k0 + q * blockDim.x;
+          const unsigned hi = hit_offset + (k < block_total ? chunk_hits[k] : 0u);
+          fits[q] = k < block_total && pos0 + k < p.track_hit_capacity && hi < T; // else flagged: a track that did not fit
+          if (!fits[q]) continue;
+          id[q] = in.id(hi);
+          x[q] = in.x(hi);
+          y[q] = in.y(hi);
+          z[q] = in.z(hi);
+        }
+#pragma unroll
+        for (unsigned q = 0; q < flight; ++q) {
+          if (!fits[q]) continue;
+          const unsigned at = pos0 + k0 + q * blockDim.x;
+          out.id(at) = id[q];
+          out.x(at) = x[q];
+          out.y(at) = y[q];
+          out.z(at) = z[q];
+        }
       }
       __syncthreads(); // chunk_hits is reused by the next chunk
       carry += block_total;
