@@ -224,10 +224,7 @@ static bool lanes_accepted(unsigned threads, unsigned lanes, unsigned ring_globa
          (threads == 512 && (lanes == 2 || lanes == 4));
 }
 
-// Retina decoding: keys of an event in L2-resident global scratch (shared memory would hold 24 KiB
-// for 3072 keys and allow six CTAs per SM instead of eight), the bucket order of up to 8192
-// clusters in shared memory (16 KiB).
-static constexpr unsigned retina_key_capacity = 0;
+// Retina decoding: the bucket order of up to 8192 clusters in shared memory (16 KiB).
 static constexpr unsigned retina_order_capacity_max = 8192;
 static constexpr size_t n_sensors_total = velo::n_sensors;
 
@@ -562,7 +559,7 @@ namespace {
       rp.container = c->sorted.p;
       rp.key_scratch = c->retina_keys.p;
       rp.status = c->status.p;
-      rp.smem_key_capacity = retina_key_capacity;
+      rp.hit_scratch = c->hit_scratch.p;
       rp.smem_order_capacity = c->retina_order_capacity;
       rp.cluster_capacity = static_cast<unsigned>(c->cap_clusters);
       VELO_CUDA(cudaMemsetAsync(c->retina_bank_index.p, 0, n_sensors * sizeof(unsigned), stream));
@@ -576,7 +573,7 @@ namespace {
       VELO_CUDA(cudaGetLastError());
       VELO_CUDA(mark());
       retina_decode_kernel<<<n, decode_threads,
-                             retina_key_capacity * sizeof(long long) + c->retina_order_capacity * sizeof(uint16_t), stream>>>(rp);
+                             c->retina_order_capacity * sizeof(uint16_t), stream>>>(rp);
       VELO_CUDA(cudaGetLastError());
       VELO_CUDA(mark());
     }
