@@ -69,6 +69,9 @@ namespace velo {
     // the event's module pairs, last first: a step's three are mps[25 - first] onwards
     ModulePair mps[n_module_pairs];
     // the seeding's h1, and their h0 candidates in pendulum order (4 or 8 places each)
+    unsigned seed_before[9];         // the window's hits to search before each of its words, and all
+    uint32_t seed_bits[8];           // those words
+    unsigned n_h0;                   // unused hits of the previous module pair
     uint16_t seed_h1[seed_slots / 4];
     uint16_t seed_h0[seed_slots];
   };
@@ -152,58 +155,51 @@ namespace velo {
 
   // The pendulum around p0 in [0, n] (SearchByTriplet.cu:351-370): step 0 is p0, step 2d - 1 is
   // p0 + d, step 2d is p0 - d, for steps below n, each position wrapping once.  As offsets from p0
-  // the visit order is 0, +1, -1, +2, ...: two words of unused hits, upwards and downwards from
-  // p0, hold the first 63 steps, and the next candidate is the nearer of their lowest bits (the
-  // upward one first).  Where those hold too few (pairs of more than 62 hits), the walk goes step
-  // by step.
+  // the visit order is 0, +1, -1, +2, ...: two words of unused hits, upwards and downwards from p0,
+  // hold 32 offsets at a time, and the next candidate is the nearer of their lowest bits, the
+  // upward one first.
   struct Pendulum {
-    uint32_t up, down; // bit d: p0 + d; bit d: p0 - 1 - d
-    unsigned k;        // candidates taken
-    __device__ __forceinline__ Pendulum(const UsedBits& used, unsigned start, unsigned n, unsigned p0) : k(0)
+    unsigned start, n, p0;
+    uint32_t up, down; // bit k: p0 + base + k; p0 - base - k
+    unsigned base;
+    __device__ __forceinline__ Pendulum(unsigned hit_start, unsigned hit_num, unsigned center) :
+      start(hit_start), n(hit_num), p0(center < hit_num ? center : 0u), up(0), down(0), base(0u - 32u)
+    {}
+    __device__ __forceinline__ void load(const UsedBits& used)
     {
-      const unsigned s = p0 < n ? p0 : 0u;
+      base += 32;
+      // offsets up to n / 2 upwards and (n - 1) / 2 downwards are visited
+      const unsigned s = p0 + base < n ? p0 + base : p0 + base - n;
       up = low_bits(used.unused(start + s), n - s);
       if (n - s < 32) up |= used.unused(start) << (n - s);
-      up = low_bits(up, n / 2 + 1);
-      if (s >= 32) {
-        down = __brev(used.unused(start + s - 32));
+      up = base <= n / 2 ? low_bits(up, n / 2 + 1 - base) : 0u;
+      const unsigned t = p0 >= base ? p0 - base : p0 + n - base;
+      if (t >= 31) {
+        down = __brev(used.unused(start + t - 31));
       }
       else {
         const uint32_t end = n >= 32 ? used.unused(start + n - 32) : used.unused(start) << (32 - n);
-        down = __brev(end) << s;
-        if (s > 0) down |= __brev(used.unused(start) << (32 - s));
+        down = (__brev(used.unused(start) << (31 - t))) | (__brev(end) << (t + 1));
       }
-      down = low_bits(down, min((n - 1) / 2, 31u));
+      down = base <= (n - 1) / 2 ? low_bits(down, (n - 1) / 2 + 1 - base) : 0u;
+      if (base == 0) down &= ~1u; // offset 0 is the upward word's
     }
     // The next candidate's position; there is one (the caller knows the number of unused hits).
-    __device__ __forceinline__ unsigned next(const UsedBits& used, unsigned start, unsigned n, unsigned p0)
+    __device__ __forceinline__ unsigned next(const UsedBits& used)
     {
-      if ((up | down) == 0) {
-        unsigned found = 0;
-        for (unsigned i = 0;; ++i) {
-          const unsigned pos = wrap(int(p0) + ((i & 1u) ? int((i + 1) / 2) : -int(i / 2)), n);
-          if (i >= n || (!used[start + pos] && found++ == k)) {
-            ++k;
-            return pos;
-          }
-        }
-      }
-      ++k;
-      const int u = up ? __ffs(up) - 1 : 64;
-      const int d = down ? __ffs(down) : 64;
-      int offset;
+      while ((up | down) == 0 && base + 32u <= n)
+        load(used);
+      const int u = up ? __ffs(up) - 1 : 32;
+      const int d = down ? __ffs(down) - 1 : 32;
+      int pos = static_cast<int>(p0);
       if (u <= d) {
-        offset = u;
+        pos += static_cast<int>(base) + u;
         up &= up - 1;
       }
       else {
-        offset = -d;
+        pos -= static_cast<int>(base) + d;
         down &= down - 1;
       }
-      return wrap(int(p0) + offset, n);
-    }
-    static __device__ __forceinline__ unsigned wrap(int pos, unsigned n)
-    {
       return static_cast<unsigned>(pos < 0 ? pos + int(n) : (pos >= int(n) ? pos - int(n) : pos));
     }
   };
@@ -323,12 +319,15 @@ namespace velo {
   }
 
   // Seeding over the current module pair (SearchByTriplet.cu:298-446).  Phase A, one thread per
-  // unused h1: its rank among the window's unused hits names it (a word of bits per lane and a
-  // bisection over their counts), and the pendulum its h0 candidates; every h1 has the same
+  // unused h1: its rank among the window's unused hits names it (a bisection over the counts of
+  // the words of bits), and the pendulum its h0 candidates; every h1 has the same
   // number of them, the unused hits of the previous module pair or n_candidates.  Phase B, one
   // thread per (h0, h1) doublet: the h2 window; the doublets of an h1 are neighbouring lanes,
   // whose shuffle reduction keeps the best (scatter, candidate order), the reference's
-  // sequential choice, and a scan queues the seeds in h1 order.  Two barriers per chunk.
+  // sequential choice, and a scan queues the seeds in h1 order.  Counting by one warp for all, and
+  // the pendulum by words of bits to its end instead of step by step where the first words hold too
+  // few unused hits, made the search 2.36 -> 2.31 ms for 16000 events and 235 -> 214 us for 10
+  // (an extra barrier costs 2 us of the former).
   // GATED kernels take the learned seed gate (gate, event-relative, or null): an unused h1
   // whose gate byte is 0 is not searched; and, for training, record each unused h1's
   // outcome (outcome: 1 no seed, 2 seed; null = off).
@@ -348,62 +347,70 @@ namespace velo {
     const ModulePair &prev = md[0], &cur = md[1], &next = md[2];
     const unsigned lane = threadIdx.x & 31u;
     const int16_t tol = static_cast<int16_t>(k.phi_tolerance_i16);
-    // the unused hits of the previous module pair
-    unsigned n_h0 = 0;
-    for (unsigned i = 32 * lane; i < prev.hit_num; i += 1024)
-      n_h0 += __popc(low_bits(used.unused(prev.hit_start + i), prev.hit_num - i));
-    n_h0 = min(__reduce_add_sync(0xFFFFFFFFu, n_h0), n_candidates);
     const unsigned places_log = n_candidates > 4 ? 3 : 2;
     for (unsigned w0 = 0; w0 < cur.hit_num; w0 += seed_window_hits) {
       const unsigned n_window = min(seed_window_hits, cur.hit_num - w0);
       const unsigned first = cur.hit_start + w0;
-      // the window's unused hits, 32 per lane of every warp
-      uint32_t word = 32 * lane < n_window ? low_bits(used.unused(first + 32 * lane), n_window - 32 * lane) : 0u;
       if constexpr (GATED) {
-        const unsigned unused = __reduce_add_sync(0xFFFFFFFFu, __popc(word));
-        if (threadIdx.x == 0) {
-          s.local_hits += unused;
-          s.candidates += unused;
-        }
         if (gate != nullptr) {
           for (unsigned i = threadIdx.x; i < (n_window + 31u) / 32u * 32u; i += blockDim.x) {
             const uint32_t pass = __ballot_sync(0xFFFFFFFFu, i < n_window && !used[first + i] && gate[first + i] != 0);
             if (lane == 0) s.pass[i / 32] = pass;
           }
           __syncthreads();
-          word = 32 * lane < n_window ? s.pass[lane] : 0u;
         }
       }
-      static_assert(seed_window_hits == 256, "the scan and the bisection are over 8 words");
-      unsigned before = __popc(word); // the hits up to this lane's word, then those before it
+      // One warp counts for all (barriers cost less than every warp's share of this): the
+      // window's unused hits, 32 per lane, and those of the previous module pair
+      if (threadIdx.x < 32) {
+        static_assert(seed_window_hits == 256, "8 words");
+        uint32_t word = 32 * lane < n_window ? low_bits(used.unused(first + 32 * lane), n_window - 32 * lane) : 0u;
+        if constexpr (GATED) {
+          const unsigned unused = __reduce_add_sync(0xFFFFFFFFu, __popc(word));
+          if (lane == 0) {
+            s.local_hits += unused;
+            s.candidates += unused;
+          }
+          if (gate != nullptr) word = 32 * lane < n_window ? s.pass[lane] : 0u;
+        }
+        unsigned before = __popc(word);
 #pragma unroll
-      for (unsigned o = 1; o < 8; o *= 2) {
-        const unsigned t = __shfl_up_sync(0xFFFFFFFFu, before, o);
-        if (lane >= o) before += t;
+        for (unsigned o = 1; o < 8; o *= 2) {
+          const unsigned t = __shfl_up_sync(0xFFFFFFFFu, before, o);
+          if (lane >= o) before += t;
+        }
+        if (lane < 8) {
+          s.seed_before[lane + 1] = before;
+          s.seed_bits[lane] = word;
+        }
+        unsigned n_h0 = 0;
+        for (unsigned i = 32 * lane; i < prev.hit_num; i += 1024)
+          n_h0 += __popc(low_bits(used.unused(prev.hit_start + i), prev.hit_num - i));
+        n_h0 = __reduce_add_sync(0xFFFFFFFFu, n_h0);
+        if (lane == 0) {
+          s.seed_before[0] = 0;
+          s.n_h0 = n_h0;
+        }
       }
-      const unsigned n_h1 = __shfl_sync(0xFFFFFFFFu, before, 7);
-      before -= __popc(word);
+      __syncthreads();
+      const unsigned n_h1 = s.seed_before[8], n_h0 = min(s.n_h0, n_candidates);
       const unsigned per_chunk = min(blockDim.x, seed_slots >> places_log);
       for (unsigned c0 = 0; c0 < n_h1; c0 += per_chunk) {
         const unsigned n_chunk = min(per_chunk, n_h1 - c0);
         // Phase A
-        if ((threadIdx.x & ~31u) < n_chunk) { // warps with work, whole
-          const unsigned rank = c0 + min(threadIdx.x, n_chunk - 1);
-          unsigned at = 0; // the last word with no more than rank hits before it
+        if (threadIdx.x < n_chunk) {
+          {
+            const unsigned rank = c0 + threadIdx.x;
+            unsigned at = 0; // the last word with no more than rank hits before it
 #pragma unroll
-          for (unsigned step = 4; step >= 1; step /= 2)
-            if (__shfl_sync(0xFFFFFFFFu, before, at + step) <= rank) at += step;
-          const uint32_t bits = __shfl_sync(0xFFFFFFFFu, word, at);
-          const unsigned offset = rank - __shfl_sync(0xFFFFFFFFu, before, at);
-          if (threadIdx.x < n_chunk) {
-            const unsigned h1 = first + 32 * at + select_bit(bits, offset);
+            for (unsigned step = 4; step >= 1; step /= 2)
+              if (s.seed_before[at + step] <= rank) at += step;
+            const unsigned h1 = first + 32 * at + select_bit(s.seed_bits[at], rank - s.seed_before[at]);
             s.seed_h1[threadIdx.x] = static_cast<uint16_t>(h1);
             if (n_h0 > 0) {
-              const unsigned p0 = static_cast<unsigned>(leftmost_hit(s, h, prev, h.phi(h1)));
-              Pendulum pendulum(used, prev.hit_start, prev.hit_num, p0);
+              Pendulum pendulum(prev.hit_start, prev.hit_num, static_cast<unsigned>(leftmost_hit(s, h, prev, h.phi(h1))));
               for (unsigned c = 0; c < n_h0; ++c)
-                s.seed_h0[(threadIdx.x << places_log) + c] =
-                  static_cast<uint16_t>(prev.hit_start + pendulum.next(used, prev.hit_start, prev.hit_num, p0));
+                s.seed_h0[(threadIdx.x << places_log) + c] = static_cast<uint16_t>(prev.hit_start + pendulum.next(used));
             }
           }
         }
@@ -467,7 +474,7 @@ namespace velo {
         }
         s.searched += n_h1;
       }
-      if (GATED && gate != nullptr && w0 + seed_window_hits < cur.hit_num) __syncthreads(); // s.pass is read
+      if (w0 + seed_window_hits < cur.hit_num) __syncthreads(); // the window's words are read
     }
   }
 
@@ -646,13 +653,23 @@ namespace velo {
     }
   }
 
-  // The bucket table of a module pair and its phi values, into its slot (a barrier follows).
-  __device__ __forceinline__ void load_pair(SearchShared& s, const Hits& h, const ModulePair& m)
+  // The phi values of a module pair into its slot, then its bucket table from them (barriers between
+  // the two and after; a larger pair's table from the records).
+  __device__ __forceinline__ void load_phi(SearchShared& s, const Hits& h, const ModulePair& m)
   {
     if (m.hit_num <= phi_capacity)
       for (unsigned i = threadIdx.x; i < m.hit_num; i += blockDim.x)
         s.phi[m.table][i] = h.phi(m.hit_start + i);
-    build_bucket_table_of(s.bucket[m.table], [h](unsigned j) { return h.phi(j); }, m.hit_start, m.hit_num);
+  }
+  __device__ __forceinline__ void build_table(SearchShared& s, const Hits& h, const ModulePair& m)
+  {
+    if (m.hit_num <= phi_capacity) {
+      const int16_t* phi = s.phi[m.table];
+      build_bucket_table_of(s.bucket[m.table], [phi](unsigned j) { return phi[j]; }, 0, m.hit_num);
+    }
+    else {
+      build_bucket_table_of(s.bucket[m.table], [h](unsigned j) { return h.phi(j); }, m.hit_start, m.hit_num);
+    }
   }
 
   // Seeding, forwarding and the tail of one event over staged hits (used bits clear):
@@ -683,7 +700,10 @@ namespace velo {
     unsigned first = n_module_pairs - 1;
     const ModulePair* md = s.mps;
     for (unsigned i = 0; i < 2; ++i)
-      load_pair(s, h, md[i]);
+      load_phi(s, h, md[i]);
+    __syncthreads();
+    for (unsigned i = 0; i < 2; ++i)
+      build_table(s, h, md[i]);
 
     // One step per module pair first = 25 ... 2 (the first without forwarding), with a single
     // copy of the seeding code.
@@ -692,7 +712,9 @@ namespace velo {
     for (;;) {
       // module pair first - 2 takes the slot of first + 1, last read by the previous step's
       // seeding before its last barrier
-      load_pair(s, h, md[2]);
+      load_phi(s, h, md[2]);
+      __syncthreads();
+      build_table(s, h, md[2]);
       const bool forward = first < n_module_pairs - 1;
       const unsigned prev_ttf = last_ttf;
       if (forward) {
