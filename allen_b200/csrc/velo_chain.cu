@@ -227,6 +227,7 @@ static bool lanes_accepted(unsigned threads, unsigned lanes, unsigned ring_globa
 // Retina decoding: the bucket order of up to 8192 clusters in shared memory (16 KiB).
 static constexpr unsigned retina_order_capacity_max = 8192;
 static constexpr size_t n_sensors_total = velo::n_sensors;
+static constexpr size_t zeroed_words = 2 * velo::n_sensors + 5; // bank index (u64), status, list and queue counters
 
 // search_by_triplet_gated_kernel instantiations (block size, ring place)
 static SearchKernel gated_search_kernel(unsigned threads, unsigned ring_global)
@@ -285,6 +286,7 @@ struct VeloChain {
   unsigned resident_few_estimate = 0, resident_few_cluster = 0, resident_few_search = 0;
 
   // workspace
+  DeviceBuffer<unsigned> zeroed; // cleared by every run: the next four lie in it
   DeviceBuffer<unsigned long long> bank_index_key;
   DeviceBuffer<unsigned> status;
   DeviceBuffer<unsigned> number_of_candidates, candidates_offsets, estimated, candidate_num, event_estimate,
@@ -407,7 +409,6 @@ namespace {
     f(c->hit_scratch, 16 * T, scratch_buffer);
     f(c->list_scratch, 2 * b.super_pixels + 64, scratch_buffer);
     f(c->lists, n, scratch_buffer);
-    f(c->list_alloc, 1, scratch_buffer);
     f(c->tracks, tracks, scratch_buffer);
     f(c->three_hit, tracks, scratch_buffer);
     f(c->three_out, tracks, scratch_buffer);
@@ -416,7 +417,6 @@ namespace {
     f(c->seed_gate, T, scratch_buffer);
     f(c->h1_outcome, T, scratch_buffer);
     f(c->gate_stats, 2 * n, scratch_buffer);
-    f(c->queue_next, 3, scratch_buffer);
     f(c->is_backward, tracks, scratch_buffer);
     f(c->retina_sizes, n * n_sensors_total, scratch_buffer);
     f(c->retina_offsets, n * n_sensors_total + 1, scratch_buffer);
@@ -523,8 +523,8 @@ namespace {
                          cudaEventRecord(ev[stage++], stream);
     };
 
-    VELO_CUDA(cudaMemsetAsync(c->bank_index_key.p, 0, n_sensors * sizeof(unsigned long long), stream));
-    VELO_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(unsigned), stream));
+    // bank index, status and the counters of list allocation and work queues
+    VELO_CUDA(cudaMemsetAsync(c->zeroed.p, 0, zeroed_words * sizeof(unsigned), stream));
     // persistent launches: claim counters at zero, events ordered by raw size (largest first)
     const bool persistent = c->persistent != 0;
     auto queue = [&](unsigned k) {
@@ -533,9 +533,6 @@ namespace {
     auto grid = [&](unsigned resident) { return persistent ? std::min(n, std::max(resident, 1u)) : n; };
     // the kernels with more registers for slices of few events (velo_kernels.cuh)
     const bool few = persistent && n <= few_events_per_sm * c->sms;
-    if (persistent) {
-      VELO_CUDA(cudaMemsetAsync(c->queue_next.p, 0, 3 * sizeof(unsigned), stream));
-    }
     if (persistent || !c->retina) {
       event_order_kernel<<<event_order_grid(n, !c->retina), scan_threads, 0, stream>>>(
         in, persistent ? c->event_order.p : nullptr, bank_index_stride(n), c->bank_index_key.p);
@@ -591,7 +588,6 @@ namespace {
       ep.list_alloc = c->list_alloc.p;
       ep.lists = c->lists.p;
       ep.queue = queue(0);
-      VELO_CUDA(cudaMemsetAsync(c->list_alloc.p, 0, sizeof(unsigned), stream));
       if (few) estimate_kernel<few_decode_threads><<<grid(c->resident_few_estimate), decode_threads, 0, stream>>>(ep);
       else estimate_kernel<2048><<<grid(c->resident_estimate), decode_threads, 0, stream>>>(ep);
       VELO_CUDA(cudaGetLastError());
@@ -695,12 +691,16 @@ namespace {
       void* args[] = {&sp};
       SearchKernel kernel = fn ? fn : v->fn;
       unsigned resident = c->resident_search;
+      unsigned smem = search_smem;
       if (few && c->resident_few_search) {
         kernel = fn ? search_by_triplet_gated_kernel<128, 1, few_events_threads> : search_by_triplet_kernel<128, 1, few_events_threads>;
         resident = c->resident_few_search;
+        // with an SM per event, its hits in shared memory too
+        if (n <= c->sms) sp.smem_hit_capacity = std::max(c->search_hit_capacity, one_event_hits);
+        smem = sp.smem_hit_capacity * search_hit_bytes;
       }
-      VELO_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(kernel), dim3(grid(resident)), dim3(c->search_threads), args,
-                                 search_smem, stream));
+      VELO_CUDA(cudaLaunchKernel(reinterpret_cast<const void*>(kernel), dim3(grid(resident)), dim3(c->search_threads), args, smem,
+                                 stream));
     }
     if (c->records) {
       // training records: the features of the candidates the search met, with its outcomes
@@ -791,7 +791,7 @@ namespace {
     const SearchKernel few_plain = search_by_triplet_kernel<128, 1, few_events_threads>,
                        few_gated = search_by_triplet_gated_kernel<128, 1, few_events_threads>;
     for (SearchKernel k : {few_plain, few_gated})
-      VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(k), search_smem));
+      VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(k), std::max(search_smem, int(one_event_hits * search_hit_bytes))));
     for (const auto& v : search_variants)
       VELO_CUDA(raise_dynamic_smem_limit(reinterpret_cast<const void*>(v.fn), search_smem));
 #define VELO_GATED_LIMIT(T, R) \
@@ -906,9 +906,12 @@ VeloStatus velo_chain_create(
   if (c->geo.reserve(1) != cudaSuccess) return cleanup(fail(VELO_ERR_CUDA, "geometry allocation failed"));
   if (cudaMemcpy(c->geo.p, &g, sizeof(g), cudaMemcpyHostToDevice) != cudaSuccess)
     return cleanup(fail(VELO_ERR_CUDA, "geometry upload failed"));
-  if (c->bank_index_key.reserve(velo::n_sensors) != cudaSuccess || c->status.reserve(1) != cudaSuccess ||
-      c->totals_dev.reserve(1) != cudaSuccess)
+  if (c->zeroed.reserve(zeroed_words) != cudaSuccess || c->totals_dev.reserve(1) != cudaSuccess)
     return cleanup(fail(VELO_ERR_CUDA, "allocation failed"));
+  c->bank_index_key.bind(c->zeroed.p, velo::n_sensors);
+  c->status.bind(c->zeroed.p + 2 * velo::n_sensors, 1);
+  c->list_alloc.bind(c->zeroed.p + 2 * velo::n_sensors + 1, 1);
+  c->queue_next.bind(c->zeroed.p + 2 * velo::n_sensors + 2, 3);
   if (cudaMallocHost(&c->totals_host, sizeof(DeviceTotals)) != cudaSuccess)
     return cleanup(fail(VELO_ERR_CUDA, "pinned allocation failed"));
   std::memset(c->totals_host, 0, sizeof(DeviceTotals));
@@ -1407,6 +1410,7 @@ void velo_chain_destroy(VeloChain* c)
     if (e) cudaEventDestroy(e);
   c->arena.release();
   c->geo.release();
+  c->zeroed.release();
   c->bank_index_key.release();
   c->status.release();
   c->number_of_candidates.release();

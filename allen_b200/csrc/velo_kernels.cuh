@@ -175,6 +175,9 @@ namespace velo {
   // events: estimate 166 -> 137 us, clustering 82 -> 70, search 437 -> 384; above that line the
   // second wave costs more (2000 events of 8200 SPs: search 1.74 ms, with 64 registers 1.87).
   constexpr unsigned few_events_threads = 1024, few_decode_threads = 1280, few_events_per_sm = 8;
+  // hits that such a search holds in shared memory with an SM per event (128 KiB): 10 events 369 -> 341
+  // us a call, 140 events 399 -> 377; with three events per SM (48 KiB each) 400 events 472 -> 497
+  constexpr unsigned one_event_hits = 8192;
   template<unsigned SM_THREADS>
   __global__ void estimate_kernel(EstimateParams p);
   template<unsigned THREADS, unsigned SM_THREADS> // 128 or 256
