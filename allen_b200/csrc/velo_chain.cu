@@ -632,6 +632,7 @@ namespace {
     sp.geo = c->geo.p;
     sp.k = c->k;
     sp.n_events = n;
+    sp.total_clusters = c->event_base.p + n;
     sp.offsets_estimated_input_size = c->offsets_est.p;
     sp.module_cluster_num = c->cluster_num.p;
     sp.sorted_container = c->sorted.p;
@@ -662,6 +663,7 @@ namespace {
     gp.geo = c->geo.p;
     gp.k = c->k;
     gp.n_events = n;
+    gp.total_clusters = c->event_base.p + n;
     gp.offsets_estimated_input_size = c->offsets_est.p;
     gp.module_cluster_num = c->cluster_num.p;
     gp.sorted_container = c->sorted.p;
@@ -719,6 +721,7 @@ namespace {
 
     ConsolidateParams kp {};
     kp.n_events = n;
+    kp.total_clusters = c->event_base.p + n;
     kp.offsets_estimated_input_size = c->offsets_est.p;
     kp.sorted_container = c->sorted.p;
     kp.tracks = c->tracks.p;
@@ -744,7 +747,7 @@ namespace {
       // the caller's containers in the half-precision layout of Allen's CUDA build
       HalfExportParams hp {};
       hp.n_events = n;
-      hp.offsets_estimated_input_size = c->offsets_est.p;
+      hp.total_clusters = c->event_base.p + n;
       hp.sorted_container = c->sorted.p;
       hp.offsets_all_velo_tracks = c->offsets_all.p;
       hp.offsets_velo_track_hit_number = c->offsets_hit_number.p;

@@ -25,7 +25,7 @@ namespace velo {
     const unsigned g0 = p.offsets_velo_tracks[e] + p.offsets_three_hit[e];
     const unsigned hit_base = p.event_track_hit_base[e];
     const unsigned TH = p.event_track_hit_base[n];
-    const unsigned T = p.offsets_estimated_input_size[n * n_module_pairs];
+    const unsigned T = *p.total_clusters;
     const unsigned hit_offset = p.offsets_estimated_input_size[e * n_module_pairs];
     const unsigned all_tracks = p.offsets_velo_tracks[n] + p.offsets_three_hit[n];
     if (T > p.cluster_capacity) return; // flagged by the clustering kernel

@@ -185,7 +185,7 @@ namespace velo {
     __shared__ unsigned kept_count;
     __shared__ std::conditional_t<RECORD, int, GateMlpShared> mlp;
     const unsigned e = blockIdx.x;
-    const unsigned T = p.offsets_estimated_input_size[p.n_events * n_module_pairs];
+    const unsigned T = *p.total_clusters;
     if (T > p.cluster_capacity) return; // flagged by the clustering kernel (before any TMEM is held)
     const unsigned* g_start = p.offsets_estimated_input_size + e * n_module_pairs;
     const unsigned* g_num = p.module_cluster_num + e * n_module_pairs;

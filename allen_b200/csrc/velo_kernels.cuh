@@ -84,11 +84,18 @@ namespace velo {
     WorkQueue queue;
   };
 
+  // The kernels behind the clustering stop when the slice needs more clusters than reserved.  They
+  // take the total from the scan of this run's event estimates (total_clusters, event_base + N): the
+  // clustering has then written neither dev_offsets_estimated_input_size nor anything else, so the
+  // last entry of that array, and every offset in it, is what an earlier run or the memory's last
+  // owner left there.
+
   // ---- search by triplet + three-hit filter, one event per CTA ----
   struct SearchParams {
     Geometry const* geo;
     Constants k;
     unsigned n_events;
+    const unsigned* total_clusters;               // T of this run (see below)
     const unsigned* offsets_estimated_input_size; // [26 N + 1]
     const unsigned* module_cluster_num;           // [26 N]
     const char* sorted_container;                 // [18 T]
@@ -125,6 +132,7 @@ namespace velo {
   // ---- copy_track_hit_number + consolidate_tracks, one event per CTA ----
   struct ConsolidateParams {
     unsigned n_events;
+    const unsigned* total_clusters;
     const unsigned* offsets_estimated_input_size;
     const char* sorted_container;
     const TrackHits* tracks;
@@ -234,7 +242,7 @@ namespace velo {
   // Velo::Clusters_t when half_t is half (backend/include/CUDABackend.h, VeloEventModel.cuh:92-189).
   struct HalfExportParams {
     unsigned n_events;
-    const unsigned* offsets_estimated_input_size;
+    const unsigned* total_clusters;
     const char* sorted_container;
     const unsigned* offsets_all_velo_tracks;
     const unsigned* offsets_velo_track_hit_number;
@@ -296,6 +304,7 @@ namespace velo {
     Geometry const* geo;
     Constants k;
     unsigned n_events;
+    const unsigned* total_clusters;
     const unsigned* offsets_estimated_input_size;
     const unsigned* module_cluster_num;
     const char* sorted_container;

@@ -778,7 +778,7 @@ namespace velo {
     const unsigned* num = p.module_cluster_num + e * n_module_pairs;
     const unsigned hit_offset = start[0];
     const unsigned n_hits = start[n_module_pairs] - hit_offset;
-    const unsigned T = p.offsets_estimated_input_size[n * n_module_pairs];
+    const unsigned T = *p.total_clusters;
     const Constants k = p.k;
     if (T > p.cluster_capacity) return; // flagged by the clustering kernel
     if (n_hits > 65536u && threadIdx.x == 0) set_error(p.status, err_hits_per_event);

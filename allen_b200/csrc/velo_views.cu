@@ -98,7 +98,7 @@ namespace velo {
   // nothing is written when an earlier stage found the slice above its bounds.
   __global__ void export_half_kernel(HalfExportParams p)
   {
-    const unsigned T = p.offsets_estimated_input_size[p.n_events * n_module_pairs];
+    const unsigned T = *p.total_clusters;
     if (T > p.cluster_capacity) return; // flagged by the clustering kernel
     const unsigned begin = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     export_elements(p.sorted_container, p.sorted_half, T, begin, stride);

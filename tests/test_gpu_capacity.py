@@ -12,7 +12,8 @@ import pytest
 
 import parity
 from allen_b200 import generator
-from allen_b200.chain import VeloError, upload
+from allen_b200 import seed_pruner
+from allen_b200.chain import COORDINATES_FP16, COORDINATES_FP32, OutputBuffersC, VeloChain, VeloError, upload
 from allen_b200.rawbanks import super_pixels_per_event
 
 pytestmark = pytest.mark.gpu
@@ -99,6 +100,48 @@ def test_workspace_too_small(chain, oracle, geometry):
     totals, out = run_chain(chain, small)
     assert totals["device_flags"] == 0
     assert parity.compare(out, oracle.run(small, geometry), small.n_events) == []
+
+
+@pytest.mark.parametrize("cfg", [dict(), dict(version=4, layout=COORDINATES_FP16), dict(retina=1), dict(learned=True)])
+def test_too_many_clusters_write_nothing(geometry, cfg):
+    """The first run on caller memory, with more clusters than it was sized for: every stage stops
+    on this run's total (the clustering has written no offsets that the later ones could read), so
+    all outputs stay as they were.  (Offsets and counts start at zero: a stage that trusted
+    them would see empty events, and write that.)"""
+    import torch
+    gen = dict(bank_version=cfg.get("version", 2), raw_format=cfg.get("retina", 0))
+    small = generator.generate(20, seed=66, mean_pileup=2.0, **gen).raw
+    big = generator.generate(20, seed=67, mean_pileup=15.0, noise_rate=1e-4, **gen).raw
+    sp = int(super_pixels_per_event(small).sum())
+    assert super_pixels_per_event(big).sum() > 3 * sp
+    layout = cfg.get("layout", COORDINATES_FP32)
+    c = VeloChain(geometry)
+    try:
+        if cfg.get("learned"):
+            seed_pruner.use_learned(c)
+        z = c.sizes(20, sp, layout)
+        ws = torch.zeros(z["workspace_bytes"] + 256, dtype=torch.uint8, device="cuda")
+        bytes_of = {
+            "dev_offsets_estimated_input_size": 4 * z["offsets_estimated_input_size"],
+            "dev_module_cluster_num": 4 * z["module_cluster_num"],
+            "dev_sorted_velo_cluster_container": z["sorted_velo_cluster_container_bytes"],
+            "dev_offsets_all_velo_tracks": 4 * z["offsets_all_velo_tracks"],
+            "dev_velo_track_hit_number": 4 * z["velo_track_hit_number"],
+            "dev_offsets_velo_track_hit_number": 4 * z["offsets_velo_track_hit_number"],
+            "dev_velo_track_hits": z["velo_track_hits_bytes"], "dev_accepted_velo_tracks": z["accepted_velo_tracks"]}
+        empty = ("dev_offsets_estimated_input_size", "dev_module_cluster_num")
+        fill = {k: 0 if k in empty else 0x5A for k in bytes_of}
+        out = {k: torch.full((n,), fill[k], dtype=torch.uint8, device="cuda") for k, n in bytes_of.items()}
+        c.bind((ws.data_ptr() + 255) & ~255, z["workspace_bytes"], 20, sp,
+               {f: out[f].data_ptr() for f, _ in OutputBuffersC._fields_}, layout)
+        c.run(upload(big))
+        with pytest.raises(VeloError) as e:
+            c.synchronize()
+        assert e.value.status == VELO_ERR_DEVICE_FLAGS and e.value.flags == ERR_INPUT_CAPACITY
+        torch.cuda.synchronize()
+        assert [k for k, t in out.items() if not bool((t == fill[k]).all())] == []
+    finally:
+        c.close()
 
 
 def test_ring_overflow_is_flagged(chain):
