@@ -294,9 +294,9 @@ struct VeloChain {
     event_track_hits, event_track_hit_base, offsets_all, track_hit_number, offsets_hit_number;
   DeviceBuffer<char> sorted, staging, track_hits, hit_scratch;
   DeviceBuffer<uint64_t> ring_scratch; // search_ring_global: one ring of 2048 entries per resident search CTA
-  DeviceBuffer<uint32_t> list_scratch; // items the estimate kernel leaves to the clustering kernel
+  DeviceBuffer<uint32_t> list_scratch; // items the estimate kernel leaves to the clustering kernel (in hit_scratch)
   DeviceBuffer<unsigned> list_alloc;   // its allocation counter
-  DeviceBuffer<uint4> lists;           // each event's part of it
+  DeviceBuffer<uint4> lists;           // each event's part of it (in retina_sizes)
   DeviceBuffer<velo::TrackHits> tracks;
   DeviceBuffer<velo::TrackletHits> three_hit, three_out;
   DeviceBuffer<uint8_t> hit_used, accepted;
@@ -407,8 +407,6 @@ namespace {
     f(c->event_track_hit_base, n + 1, scratch_buffer);
     f(c->staging, 24 * T, scratch_buffer);
     f(c->hit_scratch, 16 * T, scratch_buffer);
-    f(c->list_scratch, 2 * b.super_pixels + 64, scratch_buffer);
-    f(c->lists, n, scratch_buffer);
     f(c->tracks, tracks, scratch_buffer);
     f(c->three_hit, tracks, scratch_buffer);
     f(c->three_out, tracks, scratch_buffer);
@@ -464,6 +462,11 @@ namespace {
       buf.bind(base + at, count);
       at += align256(count * sizeof(typename std::decay_t<decltype(buf)>::value_type));
     });
+    // The item list lives from the estimate to the clustering, in memory that only the search and the
+    // retina front end write: the workspace holds nothing for it, and it has room for four times
+    // the super pixels reserved (two words each), since a slice is admitted by its clusters.
+    c->list_scratch.bind(c->hit_scratch.p, c->hit_scratch.n / sizeof(uint32_t));
+    c->lists.bind(c->retina_sizes.p, b.n);
     c->cap_events = unsigned(b.n);
     c->cap_clusters = b.T;
     c->cap_tracks = b.tracks;

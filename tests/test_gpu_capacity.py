@@ -102,6 +102,18 @@ def test_workspace_too_small(chain, oracle, geometry):
     assert parity.compare(out, oracle.run(small, geometry), small.n_events) == []
 
 
+@pytest.mark.parametrize("version", [2, 4])
+def test_more_super_pixels_than_reserved(chain, oracle, geometry, version):
+    """A slice of more super pixels than reserved whose clusters fit (two are reserved per super
+    pixel, 0.9 made) runs like any other: bit for bit the oracle's, no flag."""
+    s = generator.generate(60, seed=68 + version, bank_version=version, pileup_min=1.0, pileup_max=15.0).raw
+    chain.reserve(s.n_events, int(0.6 * super_pixels_per_event(s).sum()))
+    chain.run(upload(s), use_graph=version == 4)
+    totals = chain.synchronize()
+    assert totals["device_flags"] == 0
+    assert parity.compare(chain.outputs_to_host(totals), oracle.run(s, geometry), s.n_events) == []
+
+
 @pytest.mark.parametrize("cfg", [dict(), dict(version=4, layout=COORDINATES_FP16), dict(retina=1), dict(learned=True)])
 def test_too_many_clusters_write_nothing(geometry, cfg):
     """The first run on caller memory, with more clusters than it was sized for: every stage stops

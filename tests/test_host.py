@@ -64,3 +64,18 @@ def test_generator_library_exports():
     header = open(os.path.join(REPO, "include", "velo_generator.h")).read()
     for n in re.findall(r"(velo_gen_\w+)\s*\(", header):
         assert hasattr(lib, n), n
+
+
+def test_workspaces_of_earlier_sizes_still_suffice():
+    """A caller's workspace, sized once for its slices, stays large enough: the scratch bytes per
+    (events, super pixels), FP32 and FP16 layout, are no more than programs have reserved so far."""
+    from allen_b200 import chain
+    lib = chain._lib()
+    reserved = {(1, 1): (29440, 32000), (1, 100): (51456, 61184), (10, 26000): (5965056, 7839488),
+                (1000, 2600000): (593947136, 781149696), (16000, 41000000): (9366174720, 12318177280),
+                (5000, 100): (18243072, 18252800)}
+    for (n, sp), most in reserved.items():
+        for layout in (chain.COORDINATES_FP32, chain.COORDINATES_FP16):
+            z = chain.SizesC()
+            assert lib.velo_chain_sizes(None, n, sp, layout, C.byref(z)) == 0
+            assert 0 < z.workspace_bytes <= most[layout], (n, sp, layout)
