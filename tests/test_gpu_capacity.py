@@ -14,7 +14,7 @@ import parity
 from allen_b200 import generator
 from allen_b200 import seed_pruner
 from allen_b200.chain import COORDINATES_FP16, COORDINATES_FP32, OutputBuffersC, VeloChain, VeloError, upload
-from allen_b200.rawbanks import super_pixels_per_event
+from allen_b200.rawbanks import RawSlice, super_pixels_per_event, to_mep
 
 pytestmark = pytest.mark.gpu
 
@@ -112,6 +112,42 @@ def test_more_super_pixels_than_reserved(chain, oracle, geometry, version):
     totals = chain.synchronize()
     assert totals["device_flags"] == 0
     assert parity.compare(chain.outputs_to_host(totals), oracle.run(s, geometry), s.n_events) == []
+
+
+def with_source_id_bit_9(s, every=1):
+    """The slice with bit 9 set in the source IDs of every `every`-th event: the channel IDs of
+    version 2 and 3 banks carry it, and it is the one bit of them that a cluster item does not hold."""
+    raw = s.raw.copy()
+    for e in range(0, s.n_events, every):
+        w = raw[int(s.offsets[e]):int(s.offsets[e + 1])].view(np.uint32)
+        n_banks = int(w[0])
+        w[2 + n_banks + w[1:1 + n_banks] // 4] |= 0x200
+    return RawSlice(raw, s.offsets, s.sizes, s.types, s.bank_version)
+
+
+@pytest.mark.parametrize("version,every,mep,gen", [
+    (2, 1, False, dict(n_events=40, pileup_min=1.0, pileup_max=15.0)),
+    (3, 2, False, dict(n_events=41, sp_order=1)),
+    (2, 1, True, dict(n_events=20)),
+    (2, 2, False, dict(n_events=4, mean_pileup=40.0)),
+    (3, 1, False, dict(n_events=30, mean_pileup=0.05, noise_rate=1e-7))])
+@pytest.mark.parametrize("threads", [128, 256])
+def test_events_without_item_list(chain, oracle, geometry, version, every, mep, gen, threads):
+    """Events whose clusters do not come from an item list, alone and beside events with one, in
+    both bank layouts, sparse, and above what is held and staged in shared memory: bit for bit the
+    oracle's."""
+    s = with_source_id_bit_9(generator.generate(seed=70 + version, bank_version=version, **gen).raw, every)
+    saved = chain.get_config()
+    try:
+        chain.configure(cluster_threads=threads, cluster_stage_capacity=1024)
+        totals, out = run_chain(chain, to_mep(s) if mep else s)
+        assert totals["device_flags"] == 0
+        assert parity.compare(out, oracle.run(s, geometry), s.n_events) == []
+        ids = parity.container_fields(out["dev_sorted_velo_cluster_container"],
+                                      totals["host_total_number_of_velo_clusters"])[0]
+        assert bool((ids >> 27 & 1).any())
+    finally:
+        chain.configure(**saved)
 
 
 @pytest.mark.parametrize("cfg", [dict(), dict(version=4, layout=COORDINATES_FP16), dict(retina=1), dict(learned=True)])

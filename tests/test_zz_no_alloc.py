@@ -127,3 +127,47 @@ def test_decode_noalloc_understated_super_pixels(geometry):
     torch.cuda.synchronize()
     assert int(status.item()) & (1 << 6)
     assert bool((off == -1).all()) and bool((num == -1).all()) and bool((cont == 0xAB).all())
+
+
+@pytest.mark.parametrize("version", [2, 4])
+def test_decode_noalloc_more_super_pixels_than_stated(geometry, version):
+    """A caller that states fewer super pixels than its banks hold, but enough for their clusters:
+    the scratch has no room for the later events' item lists, and their clusters are the same."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from allen_b200 import generator
+    from allen_b200.chain import VeloChain, upload, _current_stream
+    from allen_b200.rawbanks import super_pixels_per_event
+
+    lib = _noalloc_lib()
+    g = generator.generate(80, seed=27 + version, bank_version=version, pileup_min=5.0, pileup_max=10.0)
+    n = g.raw.n_events
+    sp = int(super_pixels_per_event(g.raw).sum())
+    stated = lib.velo_noalloc_max_clusters() // 2
+    assert stated < 0.8 * sp
+    d = upload(g.raw)
+    off = torch.zeros(26 * n + 1, dtype=torch.int32, device="cuda")
+    num = torch.zeros(26 * n, dtype=torch.int32, device="cuda")
+    cont = torch.zeros(18 * 2 * stated, dtype=torch.uint8, device="cuda")
+    status = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    st = lib.velo_decode_noalloc(geometry, len(geometry), C.byref(d.c_struct()), stated, _current_stream(),
+                                 off.data_ptr(), num.data_ptr(), cont.data_ptr(), cont.numel(), status.data_ptr())
+    assert st == 0, lib.velo_noalloc_last_error_string().decode()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    chain = VeloChain(geometry)
+    try:
+        chain.reserve_for(g.raw)
+        chain.run(d)
+        ref = chain.outputs_to_host(chain.synchronize())
+    finally:
+        chain.close()
+    got_off, got_num = off.cpu().numpy().view(np.uint32), num.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got_off, ref["dev_offsets_estimated_input_size"])
+    assert np.array_equal(got_num, ref["dev_module_cluster_num"])
+    T = int(got_off[-1])
+    mask = parity.sorted_container_mask(got_off, got_num, T)
+    for a, b in zip(parity.container_fields(cont.cpu().numpy()[:18 * T], T),
+                    parity.container_fields(ref["dev_sorted_velo_cluster_container"], T)):
+        assert np.array_equal(parity._u8(a[mask]), parity._u8(b[mask]))
