@@ -296,7 +296,7 @@ struct VeloChain {
   DeviceBuffer<uint64_t> ring_scratch; // search_ring_global: one ring of 2048 entries per resident search CTA
   DeviceBuffer<uint32_t> list_scratch; // items the estimate kernel leaves to the clustering kernel (in hit_scratch)
   DeviceBuffer<unsigned> list_alloc;   // its allocation counter
-  DeviceBuffer<uint4> lists;           // each event's part of it (in retina_sizes)
+  DeviceBuffer<velo::ItemList> lists;  // each event's part of it (in retina_sizes)
   DeviceBuffer<velo::TrackHits> tracks;
   DeviceBuffer<velo::TrackletHits> three_hit, three_out;
   DeviceBuffer<uint8_t> hit_used, accepted;
@@ -466,6 +466,7 @@ namespace {
     // retina front end write: the workspace holds nothing for it, and it has room for four times
     // the super pixels reserved (two words each), since a slice is admitted by its clusters.
     c->list_scratch.bind(c->hit_scratch.p, c->hit_scratch.n / sizeof(uint32_t));
+    static_assert(sizeof(velo::ItemList) <= n_sensors_total * sizeof(unsigned), "an event's list fits its retina sizes");
     c->lists.bind(c->retina_sizes.p, b.n);
     c->cap_events = unsigned(b.n);
     c->cap_clusters = b.T;

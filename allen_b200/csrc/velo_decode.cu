@@ -520,10 +520,33 @@ namespace velo {
   // address and (version 4) sensor bit, with the bank's sensor (pair) and which of its two
   // clusters: versions 2 and 3 which << 23 | sensor << 24, version 4 pair << 24 | which << 31.
   // Candidate's cluster: two words, the column sum | pixel count << 24 and the row sum | sensor << 24.
+  // Bit 9 of a version 2 or 3 source ID, which the channel IDs of isolated SPs take over, has no room
+  // here: the list has a bit per sensor for it (note_bit_9).
   __device__ __forceinline__ uint32_t isolated_item(uint32_t word, unsigned source_id, bool v23, unsigned which)
   {
     return v23 ? (word & 0x7FFFFFu) | (which << 23) | (source_id << 24) :
                  (word & 0xFFFFFFu) | ((source_id & 0x7Fu) << 24) | (which << 31);
+  }
+
+  // Notes in the list which sensors' banks have bit 9 of the source ID set; a sensor with banks of
+  // both kinds takes the event its list.  masks: 16 words of shared memory.  Ends with a __syncthreads().
+  __device__ __noinline__ void note_bit_9(const BankTable& bt, ItemList& list, unsigned& list_at, uint32_t* masks)
+  {
+    uint32_t *with = masks, *without = masks + 8;
+    if (threadIdx.x < 16) masks[threadIdx.x] = 0;
+    __syncthreads();
+    for (unsigned b = threadIdx.x; b < bt.n_banks; b += blockDim.x) {
+      const unsigned sensor = bt.source_id[b] & 0x1FFu;
+      if (bt.flat[b] == bt.flat[b + 1] || sensor >= n_sensors) continue;
+      atomicOr(((bt.source_id[b] & 0x200u) ? with : without) + sensor / 32, 1u << (sensor & 31u));
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+      list.bit_9[threadIdx.x] = with[threadIdx.x];
+      if (with[threadIdx.x] & without[threadIdx.x]) list_at = no_item_list;
+      if (threadIdx.x == 0) list.words |= 1u;
+    }
+    __syncthreads();
   }
 
   // ------------------------------------------------------------------------------------
@@ -539,7 +562,7 @@ namespace velo {
     __shared__ uint16_t queue[estimate_queue];
     __shared__ uint16_t candidates[2 * estimate_queue]; // SP in the chunk, pixel << 10
     __shared__ unsigned queue_count[2], chunk_candidates[2];
-    __shared__ unsigned list_at, no_list;
+    __shared__ unsigned list_at;
     // the event's SPs in bank order, when they fit: the words, with the bank as its distance
     // from the hint (127: too far) in bits 24 to 30, which SPs do not use
     __shared__ uint32_t held[estimate_words + 8]; // (8: scans read on)
@@ -548,7 +571,7 @@ namespace velo {
     const int version = p.in.bank_version;
     const bool v23 = version == 2 || version == 3;
     if (threadIdx.x < 32) est_mp[threadIdx.x] = 0;
-    if (threadIdx.x == 0) cand_count = isolated_count = grown_count = no_list = 0;
+    if (threadIdx.x == 0) cand_count = isolated_count = grown_count = 0;
     if (threadIdx.x < 2) queue_count[threadIdx.x] = chunk_candidates[threadIdx.x] = 0;
 
     const EventWords ew = event_words(p.in, ev);
@@ -575,9 +598,13 @@ namespace velo {
         const unsigned at = atomicAdd(p.list_alloc, room);
         if (at <= p.list_capacity && room <= p.list_capacity - at) list_at = at;
         else atomicSub(p.list_alloc, room); // a smaller event may still fit
+        p.lists[e].words = room;
       }
     }
-    __syncthreads();
+    bool bit_9 = false;
+    for (unsigned b = threadIdx.x; v23 && b < bt.n_banks; b += blockDim.x)
+      bit_9 |= (bt.source_id[b] & 0x200u) != 0;
+    if (__syncthreads_or(bit_9) && p.lists != nullptr) note_bit_9(bt, p.lists[e], list_at, warp_sums);
     uint32_t* list = list_at != no_item_list ? p.list_scratch + list_at : nullptr;
 
     // Three passes per chunk of SPs, so that the warps do not diverge between the isolated SPs
@@ -626,9 +653,6 @@ namespace velo {
         const unsigned below = (1u << lane) - 1u;
         if (other) queue[first_queued + __popc(rest & below)] = static_cast<uint16_t>(f - chunk_base);
         if (clusters && list != nullptr) {
-          // the sensor field of a version 2 or 3 channel id takes bit 9 of the source ID too, which
-          // an item has no room for
-          if (v23 && (source_id & 0x200u)) no_list = 1;
           const unsigned k = first + __popc(one & below), k2 = first + __popc(one) + __popc(two & below);
           if (k < room) list[k] = isolated_item(word, source_id, v23, 0);
           if (clusters > 1 && k2 < room) list[k2] = isolated_item(word, source_id, v23, 1);
@@ -706,9 +730,12 @@ namespace velo {
         p.event_estimate[e] = sum;
         p.number_of_candidates[e] = 2 * bt.count_total;
         p.module_candidate_num[e] = cand_count;
-        if (p.lists != nullptr)
-          p.lists[e] = make_uint4(
-            !no_list && isolated_count + 2 * grown_count <= room ? list_at : no_item_list, room, isolated_count, grown_count);
+        if (p.lists != nullptr) {
+          ItemList& l = p.lists[e];
+          l.first = isolated_count + 2 * grown_count <= room ? list_at : no_item_list;
+          l.isolated = isolated_count;
+          l.grown = grown_count;
+        }
       }
     }
   }
@@ -756,6 +783,7 @@ namespace velo {
     unsigned region[n_module_pairs + 1]; // estimated start of each module pair, event-relative
     unsigned n_staged;
     unsigned warp_sums[33];
+    uint32_t bit_9[8]; // of the event's item list
   };
 
   // Makes clusters and appends them to the event's staging.
@@ -794,7 +822,7 @@ namespace velo {
   };
 
   // The clusters of an event without an item list (its list found no room, two clusters from
-  // too many of its SPs, or source IDs an item cannot hold): a thread per SP.  A warp takes
+  // too many of its SPs, or a sensor with banks with and without bit 9 in the source ID): a thread per SP.  A warp takes
   // fallback_banks banks at a time, whose places its first lanes hold, and walks their SPs as one
   // run.  (4000 events of 2500 SPs without lists, the whole chain: 2.06 ms; with a thread per bank,
   // its SPs one after the other, 2.92; with lists 1.19.)
@@ -910,18 +938,25 @@ namespace velo {
     char* stage_base = staged_in_smem ? reinterpret_cast<char*>(dsmem) : p.staging + ((size_t(24) * base + 15) & ~size_t(15));
     const StagedClusters st {stage_base, est_total};
 
-    const uint4 items = p.lists != nullptr ? p.lists[e] : make_uint4(no_item_list, 0, 0, 0);
+    const uint4 items = p.lists != nullptr ? *reinterpret_cast<const uint4*>(p.lists + e) : make_uint4(no_item_list, 0, 0, 0);
+    const unsigned list_words = items.y & ~1u;
     if (items.x != no_item_list) {
       // the isolated SPs from the front, the candidates' clusters from the end
       const ClusterMaker make {p, st, s, bucket, est_total};
       const uint32_t* list = p.list_scratch + items.x;
-      const bool v23 = p.in.bank_version == 2 || p.in.bank_version == 3;
+      const bool v23 = p.in.bank_version == 2 || p.in.bank_version == 3, bit_9 = items.y & 1u;
+      if (bit_9) {
+        if (threadIdx.x < 8) s.bit_9[threadIdx.x] = p.lists[e].bit_9[threadIdx.x];
+        __syncthreads();
+      }
       for (unsigned q = threadIdx.x; q < items.z; q += blockDim.x) {
         const uint32_t item = __ldcs(list + q);
-        if (v23) make.isolated(item & 0x7FFFFFu, item >> 24, (item >> 23) & 1u);
-        else make.isolated(item & 0xFFFFFFu, (item >> 24) & 0x7Fu, item >> 31);
+        unsigned source_id = item >> 24;
+        if (bit_9) source_id |= ((s.bit_9[source_id / 32] >> (source_id & 31u)) & 1u) << 9;
+        if (v23) make.isolated(item & 0x7FFFFFu, source_id, (item >> 23) & 1u);
+        else make.isolated(item & 0xFFFFFFu, source_id & 0x7Fu, item >> 31);
       }
-      const uint2* grown = reinterpret_cast<const uint2*>(list + items.y) - 1;
+      const uint2* grown = reinterpret_cast<const uint2*>(list + list_words) - 1;
       for (unsigned q = threadIdx.x; q < items.w; q += blockDim.x) {
         const uint2 g = __ldcs(grown - q);
         make.grown(g.x & 0xFFFFFFu, g.y & 0xFFFFFFu, g.x >> 24, g.y >> 24);
@@ -1006,7 +1041,7 @@ namespace velo {
     // the event's slices of the global staging and of the item list are dead
     __syncthreads();
     if (!staged_in_smem) discard_l2(stage_base, size_t(22) * est_total);
-    if (items.x != no_item_list) discard_l2(p.list_scratch + items.x, size_t(4) * items.y);
+    if (items.x != no_item_list) discard_l2(p.list_scratch + items.x, size_t(4) * list_words);
   }
 
   // Issue- and latency-bound.  16000 events of 2540 SPs: 0.65 ms, of which making the clusters 0.2

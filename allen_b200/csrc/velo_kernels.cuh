@@ -44,6 +44,16 @@ namespace velo {
   }
 
   // ---- decoding: velo_calculate_number_of_candidates + velo_estimate_input_size ----
+  // Where an event's items lie, from the estimate kernel to the clustering kernel.
+  constexpr unsigned no_item_list = 0xFFFFFFFFu;
+  struct ItemList {
+    unsigned first;    // first word in the scratch (no_item_list: no room, or too many)
+    unsigned words;    // an even number; bit 0: bit_9 counts
+    unsigned isolated; // items from the front, a word each
+    unsigned grown;    // items from the end, two words each
+    uint32_t bit_9[8]; // version 2 and 3: the sensors whose source ID has bit 9 set
+  };
+
   struct EstimateParams {
     RawInput in;
     unsigned* estimated_input_size;       // [26 N] dev_estimated_input_size
@@ -58,11 +68,9 @@ namespace velo {
     uint32_t* list_scratch;
     unsigned list_capacity;
     unsigned* list_alloc;
-    uint4* lists; // [N] first word (no_item_list: no room, or too many), words, isolated items, grown clusters
+    ItemList* lists; // [N]
     WorkQueue queue;
   };
-
-  constexpr unsigned no_item_list = 0xFFFFFFFFu;
 
   // ---- masked clustering + phi + sort by phi, one event per CTA ----
   struct ClusterSortParams {
@@ -77,7 +85,7 @@ namespace velo {
     char* sorted_container;                     // [18 T]     dev_sorted_velo_cluster_container
     char* staging;                              // [24 T]     fallback staging for large events
     const uint32_t* list_scratch;               // the estimate kernel's items
-    const uint4* lists;                         // [N] where an event's items lie (null: no lists)
+    const ItemList* lists;                      // [N] (null: no lists)
     unsigned* status;
     unsigned smem_cluster_capacity;             // clusters staged in shared memory per event
     unsigned cluster_capacity;                  // allocated T of the containers

@@ -54,7 +54,7 @@ namespace {
   constexpr size_t off_staging = align256(off_candidates_offsets + size_t(max_events + 1) * 4);
   constexpr size_t off_list = align256(off_staging + size_t(24) * max_clusters);
   constexpr size_t off_lists = align256(off_list + size_t(4) * max_clusters);
-  constexpr size_t scratch_bytes = align256(off_lists + size_t(max_events) * sizeof(uint4));
+  constexpr size_t scratch_bytes = align256(off_lists + size_t(max_events) * sizeof(velo::ItemList));
   static_assert(scratch_bytes <= 8u * 1024 * 1024, "scratch array above its stated 8 MiB");
 
   constexpr unsigned cluster_stage_capacity = 3072;
@@ -185,7 +185,7 @@ VeloStatus velo_decode_noalloc(
   ep.list_scratch = reinterpret_cast<uint32_t*>(scratch + off_list);
   ep.list_capacity = max_clusters;
   ep.list_alloc = reinterpret_cast<unsigned*>(scratch + off_list_alloc);
-  ep.lists = reinterpret_cast<uint4*>(scratch + off_lists);
+  ep.lists = reinterpret_cast<ItemList*>(scratch + off_lists);
   event_order_kernel<<<event_order_grid(n, true), scan_threads, 0, stream>>>(in, nullptr, bank_index_stride(n), bank_index);
   estimate_kernel<2048><<<n, decode_threads, 0, stream>>>(ep);
 

@@ -114,15 +114,38 @@ def test_more_super_pixels_than_reserved(chain, oracle, geometry, version):
     assert parity.compare(chain.outputs_to_host(totals), oracle.run(s, geometry), s.n_events) == []
 
 
+def event_words(s, raw, e):
+    """(u32 view of event e's words in raw, word index of each bank's source ID)"""
+    w = raw[int(s.offsets[e]):int(s.offsets[e + 1])].view(np.uint32)
+    n_banks = int(w[0])
+    return w, 2 + n_banks + w[1:1 + n_banks] // 4
+
+
 def with_source_id_bit_9(s, every=1):
     """The slice with bit 9 set in the source IDs of every `every`-th event: the channel IDs of
     version 2 and 3 banks carry it, and it is the one bit of them that a cluster item does not hold."""
     raw = s.raw.copy()
     for e in range(0, s.n_events, every):
-        w = raw[int(s.offsets[e]):int(s.offsets[e + 1])].view(np.uint32)
-        n_banks = int(w[0])
-        w[2 + n_banks + w[1:1 + n_banks] // 4] |= 0x200
+        w, source = event_words(s, raw, e)
+        w[source] |= 0x200
     return RawSlice(raw, s.offsets, s.sizes, s.types, s.bank_version)
+
+
+def with_two_banks_of_a_sensor(s):
+    """(The slice with a bank of isolated super pixels, in each event that has one, renamed to the
+    last bank's sensor with bit 9 set, the number of such events): the one sensor then has banks
+    with and without the bit, which an item list cannot tell apart.  (No candidates, which would be
+    looked up in the sensor's last bank.)"""
+    raw, renamed = s.raw.copy(), 0
+    for e in range(s.n_events):
+        w, source = event_words(s, raw, e)
+        for at in source[:-1]:
+            words = w[at + 2:at + 2 + w[at + 1]]
+            if len(words) and bool((words >> 31).all()) and w[source[-1] + 1]:
+                w[at] = w[source[-1]] | 0x200
+                renamed += 1
+                break
+    return RawSlice(raw, s.offsets, s.sizes, s.types, s.bank_version), renamed
 
 
 @pytest.mark.parametrize("version,every,mep,gen", [
@@ -130,22 +153,26 @@ def with_source_id_bit_9(s, every=1):
     (3, 2, False, dict(n_events=41, sp_order=1)),
     (2, 1, True, dict(n_events=20)),
     (2, 2, False, dict(n_events=4, mean_pileup=40.0)),
-    (3, 1, False, dict(n_events=30, mean_pileup=0.05, noise_rate=1e-7))])
+    (3, 1, False, dict(n_events=30, mean_pileup=0.05, noise_rate=1e-7)),
+    (2, 0, False, dict(n_events=40, pileup_min=0.5, pileup_max=3.0)),
+    (3, 0, False, dict(n_events=41, mean_pileup=1.0))])
 @pytest.mark.parametrize("threads", [128, 256])
-def test_events_without_item_list(chain, oracle, geometry, version, every, mep, gen, threads):
-    """Events whose clusters do not come from an item list, alone and beside events with one, in
-    both bank layouts, sparse, and above what is held and staged in shared memory: bit for bit the
-    oracle's."""
-    s = with_source_id_bit_9(generator.generate(seed=70 + version, bank_version=version, **gen).raw, every)
+def test_source_id_bit_9(chain, oracle, geometry, version, every, mep, gen, threads):
+    """Source IDs with bit 9 set, in all events and beside events without, in both bank layouts,
+    sparse, and above what is held and staged in shared memory; and (every = 0) a sensor with banks of
+    both kinds, whose event has no item list: bit for bit the oracle's."""
+    s = generator.generate(seed=70 + version, bank_version=version, **gen).raw
+    if every:
+        s = with_source_id_bit_9(s, every)
+    else:
+        s, renamed = with_two_banks_of_a_sensor(s)
+        assert renamed > s.n_events // 4
     saved = chain.get_config()
     try:
         chain.configure(cluster_threads=threads, cluster_stage_capacity=1024)
         totals, out = run_chain(chain, to_mep(s) if mep else s)
         assert totals["device_flags"] == 0
         assert parity.compare(out, oracle.run(s, geometry), s.n_events) == []
-        ids = parity.container_fields(out["dev_sorted_velo_cluster_container"],
-                                      totals["host_total_number_of_velo_clusters"])[0]
-        assert bool((ids >> 27 & 1).any())
     finally:
         chain.configure(**saved)
 
