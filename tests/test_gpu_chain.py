@@ -6,6 +6,7 @@ import golden_io
 import parity
 from allen_b200 import generator
 from allen_b200.chain import VeloError, upload
+from allen_b200.rawbanks import super_pixels_per_event
 
 pytestmark = pytest.mark.gpu
 
@@ -102,15 +103,15 @@ def test_host_pipeline_matches_oracle(oracle, geometry):
         assert np.array_equal(out["dev_velo_track_hits_id_xyz"], parity._u8(ref["dev_velo_track_hits"])[:16 * TH])
 
 
-@pytest.mark.parametrize("threads,lanes", [(128, 1), (256, 2), (256, 4), (512, 4), (128, 0), (256, 0), (512, 0)])
-def test_search_variants_identical(chain, oracle, geometry, threads, lanes):
-    """Every compiled search configuration gives the same bit-exact result (one CTA per event,
+@pytest.mark.parametrize("threads", [128, 256, 512])
+def test_search_variants_identical(chain, oracle, geometry, threads):
+    """Every block size of the search gives the same bit-exact result (one CTA per event,
     rings in shared memory; the tuned configuration's persistent launches with global rings are
     what every other test runs)."""
     g = generator.generate(40, seed=77, pileup_min=1.0, pileup_max=15.0)
     saved = chain.get_config()
     try:
-        chain.configure(search_threads=threads, search_lanes_per_seed=lanes, search_hit_capacity=2048,
+        chain.configure(search_threads=threads, search_lanes_per_seed=0, search_hit_capacity=2048,
                         cluster_stage_capacity=2048, search_ring_global=0, persistent=0)
         totals, out = run_chain(chain, g.raw)
         assert totals["device_flags"] == 0
@@ -119,17 +120,51 @@ def test_search_variants_identical(chain, oracle, geometry, threads, lanes):
         chain.configure(**saved)
 
 
-@pytest.mark.parametrize("blob", [65536, 16384, 4096])
-def test_decode_staging_paths(chain, oracle, geometry, blob):
-    """Raw-event staging sizes that select each decoding path: the event and its sorted
-    bank copies in shared memory (64 KiB), the event alone with the full neighbour scans
-    (16 KiB, events of about 13 KB), and the event read from global memory (4 KiB)."""
-    g = generator.generate(40, seed=31, pileup_min=1.0, pileup_max=15.0)
+def test_settings_without_effect_are_taken(chain, oracle, geometry):
+    """Lanes per seed candidate and raw-event staging sizes choose nothing, and are accepted and
+    refused as ever: the values that a configuration file may hold run, the others do not."""
+    g = generator.generate(20, seed=84, pileup_min=1.0, pileup_max=15.0)
+    ref = oracle.run(g.raw, geometry)
+    saved = chain.get_config()
+    flat = dict(search_ring_global=0, persistent=0)
+    try:
+        for threads, lanes in ((128, 1), (128, 2), (256, 1), (256, 2), (256, 4), (512, 2), (512, 4)):
+            chain.configure(search_threads=threads, search_lanes_per_seed=lanes, **flat)
+            assert chain.get_config()["search_lanes_per_seed"] == lanes
+            totals, out = run_chain(chain, g.raw)
+            assert totals["device_flags"] == 0 and parity.compare(out, ref, g.raw.n_events) == []
+        for threads, lanes in ((64, 0), (128, 4), (512, 1), (256, 3)):
+            with pytest.raises(VeloError):
+                chain.configure(search_threads=threads, search_lanes_per_seed=lanes, **flat)
+        with pytest.raises(VeloError):
+            chain.configure(search_threads=128, search_lanes_per_seed=1, search_ring_global=1, persistent=1)
+        chain.configure(**saved)
+        chain.configure(estimate_blob_bytes=65536, cluster_blob_bytes=32768)
+        totals, out = run_chain(chain, g.raw)
+        assert totals["device_flags"] == 0 and parity.compare(out, ref, g.raw.n_events) == []
+        for bad in (dict(estimate_blob_bytes=1 << 20), dict(cluster_blob_bytes=1 << 20), dict(cluster_blob_bytes=8)):
+            with pytest.raises(VeloError):
+                chain.configure(**bad)
+    finally:
+        chain.configure(**saved)
+
+
+@pytest.mark.parametrize("threads", [128, 256])
+@pytest.mark.parametrize("capacity", [0, 1024, 8192])
+@pytest.mark.parametrize("version", [2, 4])
+def test_decode_paths(chain, oracle, geometry, capacity, threads, version):
+    """Events on both sides of the 3584 super pixels that the estimate kernel holds in shared memory,
+    their clusters staged in shared memory (8192), in global memory (0: all but the smallest) or some
+    of each (1024), by blocks of both sizes: the same results, bit for bit."""
+    g = generator.generate(24, seed=31, bank_version=version, pileup_min=1.0, pileup_max=25.0)
+    sp = super_pixels_per_event(g.raw)
+    assert sp.min() < 3584 < sp.max()
     saved = chain.get_config()
     try:
-        chain.configure(estimate_blob_bytes=blob, cluster_blob_bytes=min(blob, 32768),
-                        cluster_stage_capacity=1024 if blob < 65536 else 2560)
-        totals, out = run_chain(chain, g.raw)
+        with pytest.raises(VeloError):
+            chain.configure(cluster_threads=64)
+        chain.configure(cluster_threads=threads, cluster_stage_capacity=capacity)
+        totals, out = run_chain(chain, g.raw, use_graph=threads == 256)
         assert totals["device_flags"] == 0
         assert parity.compare(out, oracle.run(g.raw, geometry), g.raw.n_events) == []
     finally:
@@ -158,23 +193,6 @@ def test_persistent_work_queue_identical(chain, oracle, geometry, claim):
     saved = chain.get_config()
     try:
         chain.configure(persistent=1, events_per_claim=claim)
-        totals, out = run_chain(chain, g.raw, use_graph=True)
-        assert totals["device_flags"] == 0
-        assert parity.compare(out, oracle.run(g.raw, geometry), g.raw.n_events) == []
-    finally:
-        chain.configure(**saved)
-
-
-@pytest.mark.parametrize("threads,blob", [(128, 0), (128, 16384), (256, 0)])
-def test_cluster_block_size_and_global_sorted_copies(chain, oracle, geometry, threads, blob):
-    """The clustering kernel with 128 or 256 threads, its sorted bank copies in shared memory
-    or (blob 0: nothing staged) in the global scratch: the same results, bit for bit."""
-    g = generator.generate(200, seed=83, pileup_min=1.0, pileup_max=15.0)
-    saved = chain.get_config()
-    try:
-        with pytest.raises(VeloError):
-            chain.configure(cluster_threads=64)
-        chain.configure(cluster_threads=threads, cluster_blob_bytes=blob)
         totals, out = run_chain(chain, g.raw, use_graph=True)
         assert totals["device_flags"] == 0
         assert parity.compare(out, oracle.run(g.raw, geometry), g.raw.n_events) == []
