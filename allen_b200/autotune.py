@@ -1,12 +1,11 @@
 """Autotuner of the chain's launch configuration.
 
-Sweeps, on a generated workload of the target occupancy, the search kernel's block size and
-lanes per seed candidate (the compiled pairs), the clustering kernel's block size, the
-shared-memory staging capacities of the search, clustering and estimate kernels, the place of the search's ring of tracks to follow, and
-persistent launches with a work queue (events claimed per CTA) against one CTA per event, by
-coordinate descent: each parameter in turn takes the
-value with the highest events/s (CUDA-event timed graph replays) while the others stay at
-the current best.  The winner is written to allen_b200/data/launch_config.json, which
+Sweeps, on a generated workload of the target occupancy, the search kernel's block size and the
+place of its ring of tracks to follow (the compiled pairs), the clustering kernel's block size, the
+shared-memory staging capacities of the search and the clustering, and persistent launches with a
+work queue (events claimed per CTA) against one CTA per event, by coordinate descent: each
+parameter in turn takes the value with the highest events/s (CUDA-event timed graph replays) while
+the others stay at the current best.  The winner is written to allen_b200/data/launch_config.json, which
 VeloChain loads by default.  tune_learned() does the same for the learned mode, with the seed
 gate's threshold and the seed window as coordinates constrained by tracking quality (run by
 allen_b200.train_seed_pruner).
@@ -20,7 +19,7 @@ import json
 import os
 import time
 
-# (block size, lanes per seed candidate, ring of tracks to follow in global scratch)
+# (block size, lanes per seed candidate - without effect -, ring of tracks to follow in global scratch)
 SEARCH_VARIANTS = [(128, 0, 0), (256, 0, 0), (512, 0, 0), (64, 0, 1), (96, 0, 1), (128, 0, 1), (256, 0, 1)]
 SEARCH_CAPACITIES = [0, 1024, 2048, 2560, 3072, 4096]
 CLUSTER_CAPACITIES = [0, 1024, 2048, 2560, 3072]
@@ -205,6 +204,8 @@ def main():
                                          pileup_max=args.pileup_max).raw)
     dev = [upload(s) for s in slices]
     chain = VeloChain(use_tuned=False)
+    # without effect, but counted against the shared memory that the other settings may take
+    chain.configure(cluster_blob_bytes=0, estimate_blob_bytes=0)
     chain.reserve(max(s.n_events for s in slices), max(int(super_pixels_per_event(s).sum()) for s in slices) + 64)
     t0 = time.time()
     best, rate, trials = tune(chain, dev)

@@ -129,11 +129,14 @@ def pin(s):
     return pin_slice(s)
 
 
-def kernel_bytes(n, raw_bytes, T, H, n4, n3_all, n3_out, TH, tracks_all):
+def kernel_bytes(n, raw_bytes, T, H, candidates, n4, n3_all, n3_out, TH, tracks_all):
     """Algorithmic bytes per launch of each kernel for one slice (no re-reads counted)."""
+    # the items that the estimate leaves to the clustering: a word per isolated super pixel's
+    # cluster, two per cluster that a candidate grew into
+    items = 4 * (T - candidates) + 8 * (H - (T - candidates))
     return {
-        "estimate_kernel": raw_bytes + 4 * (N_MP * n + 3 * n),
-        "cluster_sort_kernel": raw_bytes + 4 * N_MP * n + 18 * H + 4 * (2 * N_MP * n + 1),
+        "estimate_kernel": raw_bytes + 4 * (N_MP * n + 3 * n) + items,
+        "cluster_sort_kernel": items + 4 * N_MP * n + 18 * H + 4 * (2 * N_MP * n + 1),
         "search_by_triplet_kernel": 18 * H + 8 * N_MP * n + T + 54 * n4 + 6 * (n3_all + n3_out) + 24 * n,
         "consolidate_kernel": 54 * n4 + 6 * n3_out + 16 * TH + 16 * TH + 4 * (2 * tracks_all + 1) + tracks_all
                               + 4 * 4 * (n + 1),
@@ -292,8 +295,10 @@ def run_ours(args):
         n = s.n_events
         cn = chain._fetch(out["dev_module_cluster_num"], 4 * N_MP * n, np.uint32)
         at = chain._fetch(out["dev_atomics_velo"], 4 * 3 * n, np.uint32).reshape(-1, 3)
+        cand = chain._fetch(out["dev_module_candidate_num"], 4 * n, np.uint32)
         raw_bytes = s.raw.nbytes + s.offsets.nbytes + s.sizes.nbytes + s.types.nbytes
         counts.append(dict(n=n, raw_bytes=raw_bytes, T=t["host_total_number_of_velo_clusters"], H=int(cn.sum()),
+                           candidates=int(cand.sum()),
                            n4=t["host_number_of_velo_tracks_at_least_four_hits"], n3_all=int(at[:, 0].sum()),
                            n3_out=t["host_number_of_three_hit_tracks_filtered"],
                            TH=t["host_accumulated_number_of_hits_in_velo_tracks"],
@@ -332,7 +337,7 @@ def run_ours(args):
     kb = [kernel_bytes(**c) for c in counts]
     per_kernel = {}
     for name, total_ms in ktimes.items():
-        if name == "kalman_filter_kernel":
+        if name in ("kalman_filter_kernel", "seed_gate_kernel"):
             continue  # not launched in the plain chain (its timing slot spans no kernel)
         avg = total_ms / max(runs, 1)
         entry = {"ms_per_launch": round(avg, 4), "share": None}
@@ -697,10 +702,9 @@ def run_ours(args):
             "roofline": roofline,
             "chain_hbm_gbs": round(chain_gbs, 1),
             "kernels": per_kernel,
-            # per slice: estimate, scan, clustering, search, scan, consolidation, totals
-            # (+ the event order of persistent launches)
-            "gpu_launches": sum(1 for v in per_kernel.values() if v["ms_per_launch"] > 0) * len(dev) * args.steps
-                            + (len(dev) * args.steps if args.events and chain.get_config().get("persistent") else 0),
+            # per slice: event order and bank index, estimate, scan, clustering, search, scan,
+            # consolidation, totals
+            "gpu_launches": (1 + sum(1 for v in per_kernel.values() if v["ms_per_launch"] > 0)) * len(dev) * args.steps,
             "clocks": clocks.summary(),
             "learned": learned,
             "kalman": kalman,
