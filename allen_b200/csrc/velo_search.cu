@@ -7,9 +7,10 @@
 //
 // Design.
 //  * The event's sorted hits are staged once as 16-byte records (x, y, z, phi and the module
-//    parity that forwarding needs), so that every hit a walk visits costs one vector load: in shared memory, or for events above the
-//    shared-memory capacity (and in the tuned launch, every event) in a global scratch
-//    slice that stays in L2, through the same code.
+//    parity that forwarding needs), so that every hit a walk visits costs one vector load: in
+//    shared memory, or for events above the shared-memory capacity (and in the tuned launch, every
+//    event of a slice of more events than SMs) in a global scratch slice that stays in L2, through
+//    the same code.
 //  * Which hits are used is a bit per hit in shared memory (the reference's hit_used).
 //  * Within a step every seed candidate (h1) and every track to follow is independent:
 //    seeding only reads the used bits, forwarding only sets them, and each track to follow
@@ -24,8 +25,9 @@
 //  * An entry of the ring of tracks to follow (2048 entries, as the reference) holds a seed's
 //    three hits, or a track's last two hits, its number and its hit count, so that forwarding
 //    reads nothing else of the track.  Tracks are written to dev_tracks as they grow.
-//  * Leftmost binary searches over a module pair's phi go through a 128-bucket table
-//    per module pair, built once per event, plus a short scan: same index, fewer loads.
+//  * Leftmost binary searches over a module pair's phi go through a 128-bucket table plus a
+//    short scan: same index, fewer loads.  A step reads the tables of three module pairs, and each
+//    step builds the one it adds in the slot of the one it leaves.
 #include <type_traits>
 
 #include "velo_kernels.cuh"
@@ -894,9 +896,10 @@ namespace velo {
   // through L2 shared memory does not limit the CTAs per SM, and the resident events hide more
   // latency than the cap costs (16000 events: 2.36 ms; twelve CTAs per SM at 40 registers 2.51,
   // eight at 64 registers 2.83).  Slices that eight CTAs per SM hold take 64 registers (128
-  // threads with global rings: 1000 events 437 -> 384 us, 10 events 245 -> 235 us).  The seeding by used bits, against used flags in the hit records,
-  // an index of the unused hits and a packed list of doublets per step (ten barriers a step
-  // instead of five): 3.01 -> 2.36 ms, 10 events 313 -> 245 us.
+  // threads with global rings: 1000 events 437 -> 384 us, 10 events 245 -> 235 us).  The seeding by
+  // used bits, against used flags in the hit records, an index of the unused hits and a packed list
+  // of doublets per step (ten barriers a step instead of five): 3.01 -> 2.36 ms, 10 events 313 ->
+  // 245 us.
   template<unsigned THREADS, unsigned RING, bool GATED>
   __device__ __forceinline__ void search_events(const SearchParams& p)
   {
@@ -919,8 +922,9 @@ namespace velo {
   }
 
   // The learned search: the seeding behind the seed gate (with seed_gate null, the plain
-  // search, recording each seed candidate's outcome when h1_outcome is set).  The gate costs
-  // one byte read per candidate, so this kernel keeps the plain kernel's register budget.
+  // search, recording each seed candidate's outcome when h1_outcome is set).  Capped like the plain
+  // kernel, though it spills more at 32 registers (244 bytes of stores and 344 of loads against 44 and
+  // 84): 4000 events 0.63 ms, the plain search 0.65.
   template<unsigned THREADS, unsigned RING, unsigned SM_THREADS>
   __global__ void __launch_bounds__(THREADS, SM_THREADS / THREADS) search_by_triplet_gated_kernel(SearchParams p)
   {

@@ -270,7 +270,7 @@ VeloStatus velo_chain_outputs(const VeloChain* chain, VeloChainOutputs* outputs)
 typedef struct {
   unsigned search_threads;
   unsigned search_lanes_per_seed;
-  unsigned search_hit_capacity;    /* hits of an event staged in shared memory (15 B each) */
+  unsigned search_hit_capacity;    /* hits of an event staged in shared memory (16 B each) */
   unsigned cluster_stage_capacity; /* clusters of an event staged in shared memory (22 B each, 64 at least) */
   unsigned cluster_blob_bytes;     /* accepted within the shared-memory limit, without effect: the decoding */
   unsigned estimate_blob_bytes;    /* kernels read each raw word once and stage no raw events */
